@@ -283,8 +283,7 @@ int ctx_set_projectors(cpw_b200_ctx* c, int nanl, const double* anlga, int ld, c
   c->xnl_h.resize(nanl);
   e = cudaMemcpyAsync(c->xnl_h.data(), dx.p, nanl * sizeof(double), cudaMemcpyDeviceToHost, c->stream);
   if (e != cudaSuccess) return cuda_fail(e, "set_projectors copy");
-  c->tc_ready = false;
-  c->oz_nl_ready = false;
+  projectors_changed(c);
   e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return cuda_fail(e, "set_projectors");
   if (c->precision == 2) return tc_prepare_projectors(c);
@@ -293,6 +292,44 @@ int ctx_set_projectors(cpw_b200_ctx* c, int nanl, const double* anlga, int ld, c
 
 static int blas_fail(cublasStatus_t st, const char* what) {
   return fail(kCublas, std::string(what) + ": cuBLAS status " + std::to_string((int)st));
+}
+
+// Whether the projector products of nb bands run as residue GEMMs (crt.cu). Their cost is mostly the X
+// planes (90 bytes per element of X in FP64, 54 in MIXED_TC) until there are enough bands to share
+// them, plus conversions and five more launches than the two GEMMs they replace: ~110 us of fixed
+// cost. Measured both ways (us, other form -> residues): FP64 ZGEMMs 17,040 -> 4,630 (88,951 plane
+// waves, 864 projectors, 480 bands), 548 -> 394 (26,529, 256, 160), 119 -> 167 (18,577, 180, 37);
+// split TF32 5,900 -> 3,110, 303 -> 278, 98 -> 115 on the same three. CPW_B200_NL_CRT=1 / 0 forces
+// either way.
+static bool crt_pays(const cpw_b200_ctx* c, int nb) {
+  // int32 sums, a grid dimension, 16-bit sums over the K splits
+  if (c->nanl > kCrtMaxProjectors || nb > 65535 || c->mtxd > 15000000 || c->crt_off) return false;
+  if (const char* v = getenv("CPW_B200_NL_CRT")) return atoi(v) != 0;
+  const double flops = 16.0 * c->mtxd * c->nanl * nb;
+  return c->precision == 2 ? nb >= 128 && flops >= 1.5e10 : nb >= 64 && flops >= 1e10;
+}
+
+// The residue GEMMs ready for nb bands: X converted, buffers allocated. Where memory does not suffice, or
+// a stream capture forbids the preparation, the products stay on the other path.
+static bool crt_ready(cpw_b200_ctx* c, int nb, cudaStream_t st) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
+  const bool free_run = cap == cudaStreamCaptureStatusNone;
+  const int L = c->precision == 2 ? 9 : 15;
+  const bool have = c->crt.L == L && c->crt.m == c->mtxd && c->crt.na == c->nanl;
+  if (!have && !free_run) return false;
+  if ((!have && crt_prepare(c->crt, c->mtxd, c->nanl, L, c->anl.p, c->anld.p, st)) ||
+      crt_reserve(c->crts, c->crt, nb, free_run)) {
+    if (free_run) {
+      cudaGetLastError();
+      c->crt.buf.release();
+      c->crts.buf.release();
+      c->crt.L = 0;
+      c->crt_off = true;
+    }
+    return false;
+  }
+  return true;
 }
 
 int ctx_hkpsi_device(cpw_b200_ctx* c, int nb, const void* psi, long long ldpsi, void* hpsi, long long ldh,
@@ -317,7 +354,8 @@ int ctx_hkpsi_device(cpw_b200_ctx* c, int nb, const void* psi, long long ldpsi, 
   // gains 0.5-1% this way and keeps both on st, so that its stage timers time each kernel alone.
   // CPW_B200_NL_OVERLAP=1 / 0 forces either way.
   const bool i8_nl = with_nl && c->nanl > 0 && c->nl_slices > 0;
-  const bool cublas_nl = with_nl && c->nanl > 0 && !i8_nl && !(c->precision == 2 && c->tc_ready);
+  const bool crt_nl = with_nl && c->nanl > 0 && !i8_nl && crt_pays(c, nb) && crt_ready(c, nb, st);
+  const bool cublas_nl = with_nl && c->nanl > 0 && !i8_nl && !crt_nl && !(c->precision == 2 && c->tc_ready);
   bool overlap = false;
   cudaEvent_t ov_t0 = nullptr, ov_t1 = nullptr;
   if (cublas_nl) {
@@ -393,6 +431,14 @@ int ctx_hkpsi_device(cpw_b200_ctx* c, int nb, const void* psi, long long ldpsi, 
       return fail(kCublas, "zgemm X D P");
     if (t2) cudaEventRecord(t2, st);
     c->timer.mark(kStNlProj, ov_t0, ov_t1);
+    c->timer.mark(kStNlExpand, t1, t2);
+    return kOk;
+  }
+  if (crt_nl) {
+    cudaEvent_t t0 = c->timer.on ? c->timer.take() : nullptr, t1 = c->timer.on ? c->timer.take() : nullptr;
+    cudaEvent_t t2 = c->timer.on ? c->timer.take() : nullptr;
+    if ((s = crt_nl_apply(c->crts, c->crt, nb, psi, ldpsi, hpsi, ldh, c->tcs.wait_ns, st, t0, t1, t2))) return s;
+    c->timer.mark(kStNlProj, t0, t1);
     c->timer.mark(kStNlExpand, t1, t2);
     return kOk;
   }

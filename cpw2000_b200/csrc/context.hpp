@@ -103,6 +103,27 @@ int oz_zgemm(OzScratch& w, bool conjA, int M, int N, int K, const void* A, long 
              double alpha, bool accumulate, void* C, long long ldc, int slices, unsigned long long wait_ns,
              cudaStream_t st, int tri = kOzFull);
 int oz_read_error(OzScratch& w);
+// projector products as residue GEMMs on the int8 tensor cores (crt.cu): X and X D converted once per
+// projector set for L moduli (L = 0: not converted), and the buffers of a call
+constexpr int kCrtMaxProjectors = 65535;      // K' of the expansion fits one int32 accumulation
+struct CrtOperands {
+  DevBuf buf;
+  int8_t* a1 = nullptr;     // in buf: planes of X and of X D, scales of their rows
+  int8_t* a2 = nullptr;
+  int* s1 = nullptr;
+  int* s2 = nullptr;
+  int m = 0, na = 0, L = 0;
+  int nkb1 = 0, nkb2 = 0, tiles1 = 0, tiles2 = 0;
+};
+struct CrtScratch {
+  DevBuf buf, err;
+};
+int crt_prepare(CrtOperands& o, int m, int na, int L, const void* anl, const void* anld, cudaStream_t st);
+int crt_reserve(CrtScratch& t, const CrtOperands& o, int nb, bool may_allocate);
+int crt_nl_apply(CrtScratch& t, const CrtOperands& o, int nb, const void* psi, long long ldpsi, void* hpsi,
+                 long long ldh, unsigned long long wait_ns, cudaStream_t st, cudaEvent_t t0, cudaEvent_t t1,
+                 cudaEvent_t t2);
+int crt_read_error(CrtScratch& t);
 int tc_error_flag(TcScratch& t);
 int tc_read_error(TcScratch& t);
 int tc_prepare_projectors(cpw_b200_ctx* c);
@@ -169,6 +190,10 @@ struct cpw_b200_ctx {
   cpwb::OzOperand oz_x, oz_xd;
   cpwb::OzOperand oz_gs[3];     // eigensolver: converged block of a Gram-Schmidt call, split once
   bool oz_nl_ready = false;
+  // residue operands of the current projectors; crt_off: they did not fit on the device
+  cpwb::CrtOperands crt;
+  cpwb::CrtScratch crts;
+  bool crt_off = false;
   long long tc_k1p = 0, tc_k2p = 0;     // K blocks (32 reals) of the projection and expansion operands
   bool tc_ready = false;
 
@@ -203,6 +228,13 @@ int ctx_set_basis(cpw_b200_ctx* c, int mtxd, const int* isort, const int* kgv, i
                   const int* kmscr);
 int ctx_set_potential(cpw_b200_ctx* c, const double* vscr, long long nscr);
 int ctx_set_projectors(cpw_b200_ctx* c, int nanl, const double* anlga, int ld, const double* xnlkb, bool on_device);
+// the projectors on the device have changed: what was derived from them is no longer valid
+inline void projectors_changed(cpw_b200_ctx* c) {
+  c->tc_ready = false;
+  c->oz_nl_ready = false;
+  c->crt.L = 0;
+  c->crt_off = false;
+}
 void ditsp_release(cpw_b200_ctx* c);
 int ctx_set_potential_spin(cpw_b200_ctx* c, const double* vscr_sp, long long mxdscr, int nsp);
 int ctx_set_projectors_spin(cpw_b200_ctx* c, int nanl, const double* anlsp, long long ld, const double* xnlkb);

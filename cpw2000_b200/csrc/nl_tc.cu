@@ -181,6 +181,8 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
 // CTA exits, always use kWaitNs: those complete on their own.
 __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, const volatile int* failed,
                                           unsigned long long limit_ns = kWaitNs) {
+  // a phase that is already complete costs no read of the timer (about a microsecond)
+  if (mbar_try(mbar, parity)) return true;
   const unsigned long long t0 = globaltimer_ns();
   for (unsigned it = 0;; ++it) {
     if (mbar_try(mbar, parity)) return true;
@@ -843,7 +845,8 @@ int tc_zgemm_nn(cpw_b200_ctx* c, int m, int n, int kk, const void* a, long long 
 
 int tc_check_error(cpw_b200_ctx* c) {
   if (int s = tc_read_error(c->tcs)) return s;
-  return oz_read_error(c->ozs);
+  if (int s = oz_read_error(c->ozs)) return s;
+  return crt_read_error(c->crts);
 }
 
 namespace tc {

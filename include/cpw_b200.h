@@ -92,8 +92,10 @@ int cpw_b200_wait_selftest(cpw_b200_ctx* ctx, long long limit_ns, void* stream);
 /* Projector products P = X^H psi and hpsi += X D P (hk_psi_nl_c16.f90:82-96) of
  * the context's H|psi> on the int8 tensor cores with `slices` 7-bit slices per
  * operand (1..8; the split of X and X D is kept until the projectors change),
- * in any precision form; 0 restores the form's default (cuBLAS FP64 ZGEMMs in
- * FP64 and MIXED, split-TF32 tensor-core GEMMs in MIXED_TC). 7 slices give
+ * in any precision form; 0 restores the form's default (FP64 and MIXED:
+ * residue GEMMs with 15 moduli for blocks large enough to pay for their
+ * conversion, else cuBLAS FP64 ZGEMMs; MIXED_TC: 9 moduli or split-TF32
+ * tensor-core GEMMs). 7 slices give
  * FP64-level products (~2^-48 of the row maxima); 4 give ~2^-27, without the
  * bias of FP32 accumulation (the integer sums are exact). */
 int cpw_b200_set_projector_slices(cpw_b200_ctx* ctx, int slices);

@@ -1,0 +1,103 @@
+"""Projector products as residue GEMMs (csrc/crt.cu) against an extended-precision product on the CPU.
+
+With V = 0 and no kinetic term H|psi> is X diag(xnlkb) X^H psi alone. The rows of the operands are rounded
+to 2^-57 (FP64 form) or 2^-34 (MIXED_TC) of their 2-norms or better, so an element of P is off by at
+most ~2^-56 |x| |psi|, sqrt(2 m) 2^-56 of a typical element, and the expansion adds sqrt(2 nanl) 2^-56:
+below 1e-14 and 1e-7 of the result's maximum for the sizes here (sqrt(2 m) <= 41).
+"""
+import numpy as np
+import pytest
+
+from cpw2000_b200 import configs
+from cpw2000_b200 import hk_psi as H
+
+pytestmark = pytest.mark.gpu
+TOL = {H.FP64: 1e-14, H.MIXED: 1e-14, H.MIXED_TC: 1e-7}
+
+
+@pytest.fixture(autouse=True)
+def residues(monkeypatch):
+    monkeypatch.setenv("CPW_B200_NL_CRT", "1")
+
+
+def _basis(name):
+    return configs.kpoint_inputs(configs.WORKLOADS[name](), 1)
+
+
+def _context(d, prec, x, xnl):
+    ctx = H.Context(0, precision=prec)
+    ctx.set_kpoint(d["mtxd"], d["isort"], d["kgv"], 0 * d["ekpg"], d["kmscr"])
+    ctx.set_potential(0 * d["vscr"])
+    ctx.set_projectors(x, xnl)
+    return ctx
+
+
+def _apply(cuda, ctx, psi):
+    import torch
+    # strides given outright: a transposed single column may report any
+    p, h = (torch.empty_strided(psi.shape, (1, psi.shape[0]), dtype=torch.complex128, device=cuda) for _ in range(2))
+    p.copy_(torch.from_numpy(psi))
+    ctx.hk_psi(p, h)
+    ctx.synchronize()
+    return h.cpu().numpy()
+
+
+def _exact(x, xnl, psi):
+    x, psi = x.astype(np.clongdouble), psi.astype(np.clongdouble)
+    return x @ (xnl.astype(np.longdouble)[:, None] * (x.conj().T @ psi))
+
+
+def _random(m, na, nb, seed):
+    rng = np.random.default_rng(seed)
+    x = np.asfortranarray((rng.standard_normal((m, na)) + 1j * rng.standard_normal((m, na)))
+                          * np.exp(-rng.uniform(0, 4, (m, 1))))
+    return x, rng.choice((-1.0, 1.0), na), rng.standard_normal((m, nb)) + 1j * rng.standard_normal((m, nb))
+
+
+# edges: one row or column, one more or less than a tile (128 rows, 16 columns, 4 bands, 256 columns),
+# one K block and a remainder of one
+@pytest.mark.parametrize("prec", [H.FP64, H.MIXED, H.MIXED_TC])
+@pytest.mark.parametrize("cell,na,nb", [("small", 1, 1), ("small", 129, 5), ("si2", 127, 16), ("si2", 128, 17),
+                                        ("si2", 257, 3), ("si2", 8, 255), ("si2", 33, 258)])
+def test_matches_extended_precision(cuda, prec, cell, na, nb):
+    d = _basis(cell)
+    x, xnl, psi = _random(d["mtxd"], na, nb, na + nb)
+    ctx = _context(d, prec, x, xnl)
+    ref = _exact(x, xnl, psi)
+    err = float(np.abs(_apply(cuda, ctx, psi) - ref).max() / np.abs(ref).max())
+    assert err < TOL[prec]
+    ctx.close()
+
+
+def test_scales_and_non_finite_bands(cuda):
+    """A band of tiny or huge numbers keeps its relative accuracy; a NaN or an infinity makes its own band
+    NaN and leaves the others as they are, to the bit."""
+    d = _basis("si2")
+    m = d["mtxd"]
+    x, xnl, psi = _random(m, 24, 7, 5)
+    ctx = _context(d, H.FP64, x, xnl)
+    clean = _apply(cuda, ctx, psi)
+    psi[:, 1] *= 2.0 ** -700
+    psi[:, 2] *= 2.0 ** 700
+    psi[:, 3] = 0.0
+    psi[m // 2, 4] = np.nan
+    psi[0, 5] = np.inf
+    got = _apply(cuda, ctx, psi)
+    assert np.array_equal(got[:, [0, 6]], clean[:, [0, 6]])
+    for band, e in ((1, 700), (2, -700)):
+        assert np.array_equal(got[:, band] * 2.0 ** e, clean[:, band])
+    assert np.all(got[:, 3] == 0)
+    assert np.isnan(got[:, 4]).all() and np.isnan(got[:, 5]).all()
+    ctx.close()
+
+
+def test_new_projectors_and_precision_replace_the_planes(cuda):
+    d = _basis("si2")
+    x, xnl, psi = _random(d["mtxd"], 20, 6, 7)
+    x2, xnl2, _ = _random(d["mtxd"], 31, 6, 8)
+    ctx = _context(d, H.FP64, x, xnl)
+    _apply(cuda, ctx, psi)
+    ctx.set_projectors(x2, xnl2)
+    ref = _exact(x2, xnl2, psi)
+    assert float(np.abs(_apply(cuda, ctx, psi) - ref).max() / np.abs(ref).max()) < TOL[H.FP64]
+    ctx.close()
