@@ -92,7 +92,7 @@ k_dens_z(LocalPlan p, int nbc, const double* __restrict__ occ, const C2<double>*
   __syncthreads();
   for (int it = tid; it < cb * n3; it += nt) {
     const int cl = it % cb, z = it / cb;
-    if (cl < ncol) rho[(size_t)z * p.plane + c0 + cl] += acc[(size_t)z * cb + cl];
+    if (cl < ncol) rho[(size_t)z * p.plane + slab_column(p, c0 + cl)] += acc[(size_t)z * cb + cl];
   }
 }
 

@@ -125,10 +125,7 @@ int plan_for_box(cpw_b200_ctx* c, const int kd[3], const int* kmscr, LocalPlan* 
   p.rowp = n1 + 1;
   const size_t cmax = max_smem_optin(c->device);
   const size_t esz = c->precision ? sizeof(C2<float>) : sizeof(C2<double>);
-  p.tcol = 32;
-  while (p.tcol > 4 && esz * ((size_t)p.ny * p.rowp + (size_t)p.n2 * p.tcol + n1 + n2) > cmax) p.tcol /= 2;
-  if (esz * ((size_t)p.ny * p.rowp + (size_t)p.n2 * p.tcol + n1 + n2) > cmax)
-    return fail(kUnsupported, "set_basis: plane does not fit in shared memory");
+  if (!plane_tile(esz, p, cmax)) return fail(kUnsupported, "set_basis: plane does not fit in shared memory");
   int smsm = 0;
   cudaDeviceGetAttribute(&smsm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, c->device);
   p.cb = column_tile(esz, p, cmax, (size_t)smsm);

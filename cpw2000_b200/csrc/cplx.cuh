@@ -224,6 +224,144 @@ template <int S, typename T> struct DFT<10, S, T> : DFTComp<2, 5, S, T> {};
 template <int S, typename T> struct DFT<12, S, T> : DFTComp<3, 4, S, T> {};
 template <int S, typename T> struct DFT<16, S, T> : DFTComp<4, 4, S, T> {};
 
+// ---------------- register DFTs with inputs known to be zero ----------------
+// Bit i of M: v[i] may be nonzero; the others are exactly zero and are not read. The sphere leaves the
+// middle half of every line empty on the usual boxes (kept indices 0..kd and n-kd..n-1, kd < n/4), so a
+// pass over r1 stride-r2 points starts from about half of them: a 12-point one from 6.
+template <bool A, bool B, typename T> __device__ __forceinline__ C2<T> addm(C2<T> a, C2<T> b) {
+  if constexpr (A && B) return a + b;
+  else if constexpr (A) return a;
+  else if constexpr (B) return b;
+  else return mk<T>(T(0), T(0));
+}
+template <bool A, bool B, typename T> __device__ __forceinline__ C2<T> subm(C2<T> a, C2<T> b) {
+  if constexpr (A && B) return a - b;
+  else if constexpr (A) return a;
+  else if constexpr (B) return mk<T>(-b.x, -b.y);
+  else return mk<T>(T(0), T(0));
+}
+
+template <unsigned M, int R, int S, typename T> struct DFTM;
+
+template <unsigned M, int S, typename T> struct DFTM<M, 1, S, T> { static __device__ __forceinline__ void run(C2<T>*) {} };
+
+template <unsigned M, int S, typename T> struct DFTM<M, 2, S, T> {
+  static __device__ __forceinline__ void run(C2<T>* v) {
+    constexpr bool m0 = M & 1, m1 = M & 2;
+    const C2<T> a = addm<m0, m1>(v[0], v[1]), b = subm<m0, m1>(v[0], v[1]);
+    v[0] = a;
+    v[1] = b;
+  }
+};
+
+template <unsigned M, int S, typename T> struct DFTM<M, 3, S, T> {
+  static __device__ __forceinline__ void run(C2<T>* v) {
+    constexpr bool m0 = M & 1, m1 = M & 2, m2 = M & 4;
+    if constexpr (!m1 && !m2) {
+      v[1] = v[2] = v[0];
+    } else {
+      constexpr K<T> h(0.866025403784438646763723170752936183);  // sqrt(3)/2
+      const C2<T> t1 = addm<m1, m2>(v[1], v[2]);
+      const C2<T> t3 = mul_iS<S, T>(kscal<T>(subm<m1, m2>(v[1], v[2]), h));
+      const C2<T> t2 = subm<m0, true>(v[0], scal<T>(t1, T(0.5)));
+      v[0] = addm<m0, true>(v[0], t1);
+      v[1] = t2 + t3;
+      v[2] = t2 - t3;
+    }
+  }
+};
+
+template <unsigned M, int S, typename T> struct DFTM<M, 4, S, T> {
+  static __device__ __forceinline__ void run(C2<T>* v) {
+    constexpr bool m0 = M & 1, m1 = M & 2, m2 = M & 4, m3 = M & 8, A = m0 || m2, B = m1 || m3;
+    const C2<T> a0 = addm<m0, m2>(v[0], v[2]), a1 = subm<m0, m2>(v[0], v[2]);
+    const C2<T> b0 = addm<m1, m3>(v[1], v[3]), b1 = mul_iS<S, T>(subm<m1, m3>(v[1], v[3]));
+    v[0] = addm<A, B>(a0, b0);
+    v[2] = subm<A, B>(a0, b0);
+    v[1] = addm<A, B>(a1, b1);
+    v[3] = subm<A, B>(a1, b1);
+  }
+};
+
+template <unsigned M, int S, typename T> struct DFTM<M, 5, S, T> {
+  static __device__ __forceinline__ void run(C2<T>* v) {
+#pragma unroll
+    for (int i = 0; i < 5; ++i)
+      if (!((M >> i) & 1)) v[i] = mk<T>(T(0), T(0));
+    DFT<5, S, T>::run(v);
+  }
+};
+
+template <unsigned M, int A, int B, int S, typename T> struct DFTCompM {
+  static constexpr unsigned sub(int n2) {
+    unsigned m = 0;
+    for (int n1 = 0; n1 < A; ++n1)
+      if ((M >> (B * n1 + n2)) & 1) m |= 1u << n1;
+    return m;
+  }
+  static constexpr unsigned second() {
+    unsigned m = 0;
+    for (int n2 = 0; n2 < B; ++n2)
+      if (sub(n2)) m |= 1u << n2;
+    return m;
+  }
+  template <int n2> static __device__ __forceinline__ void first(const C2<T>* v, C2<T>* t) {
+    if constexpr (n2 < B) {
+      if constexpr (sub(n2) != 0) {
+        constexpr int R = A * B;
+        constexpr ct::Tw<R> tw{};
+        C2<T> u[A];
+#pragma unroll
+        for (int n1 = 0; n1 < A; ++n1) u[n1] = v[B * n1 + n2];
+        DFTM<sub(n2), A, S, T>::run(u);
+#pragma unroll
+        for (int k1 = 0; k1 < A; ++k1) {
+          const int m = (n2 * k1) % R;
+          if (m == 0) {
+            t[k1 * B + n2] = u[k1];
+          } else if (4 * m == R) {                 // W = i*S
+            t[k1 * B + n2] = mul_iS<S, T>(u[k1]);
+          } else if (2 * m == R) {                 // W = -1
+            t[k1 * B + n2] = mk<T>(-u[k1].x, -u[k1].y);
+          } else if (4 * m == 3 * R) {             // W = -i*S
+            t[k1 * B + n2] = mul_iS<-S, T>(u[k1]);
+          } else {
+            t[k1 * B + n2] = kcmul(u[k1], K<T>(tw.c[m]), K<T>(S * tw.s[m]));
+          }
+        }
+      }
+      first<n2 + 1>(v, t);
+    }
+  }
+  static __device__ __forceinline__ void run(C2<T>* v) {
+    C2<T> t[A * B];
+    first<0>(v, t);
+#pragma unroll
+    for (int k1 = 0; k1 < A; ++k1) {
+      C2<T> u[B];
+#pragma unroll
+      for (int n2 = 0; n2 < B; ++n2) u[n2] = t[k1 * B + n2];
+      DFTM<second(), B, S, T>::run(u);
+#pragma unroll
+      for (int k2 = 0; k2 < B; ++k2) v[k1 + A * k2] = u[k2];
+    }
+  }
+};
+template <unsigned M, int S, typename T> struct DFTM<M, 6, S, T> : DFTCompM<M, 2, 3, S, T> {};
+template <unsigned M, int S, typename T> struct DFTM<M, 8, S, T> : DFTCompM<M, 2, 4, S, T> {};
+template <unsigned M, int S, typename T> struct DFTM<M, 9, S, T> : DFTCompM<M, 3, 3, S, T> {};
+template <unsigned M, int S, typename T> struct DFTM<M, 10, S, T> : DFTCompM<M, 2, 5, S, T> {};
+template <unsigned M, int S, typename T> struct DFTM<M, 12, S, T> : DFTCompM<M, 3, 4, S, T> {};
+template <unsigned M, int S, typename T> struct DFTM<M, 16, S, T> : DFTCompM<M, 4, 4, S, T> {};
+
+// The kept indices of a line n = r (n / r) lie in its first and last quarter(r) blocks of n / r points
+// when kd < quarter(r) (n / r) (r = 1: first and last block are the same one).
+__host__ __device__ constexpr int quarter(int r) { return (r + 3) / 4; }
+__host__ __device__ constexpr bool in_quarters(int kd, int r, int rest) { return r > 1 && kd < quarter(r) * rest; }
+__host__ __device__ constexpr unsigned quarter_bits(int r) {
+  return ((1u << quarter(r)) - 1) | (((1u << quarter(r)) - 1) << (r - quarter(r)));
+}
+
 // Radices the runtime dispatch accepts (a line length n is split n = r1*r2).
 __host__ __device__ constexpr bool radix_ok(int r) {
   return r == 1 || r == 2 || r == 3 || r == 4 || r == 5 || r == 6 || r == 8 || r == 9 ||

@@ -1,10 +1,10 @@
 // Kernel templates A, B, C of the local H|psi> (design in hkpsi_local.cuh).
 //
-// Template parameters fix the radix pair of each dimension (RX1*RX2 = n1,
-// RY1*RY2 = n2, RZ1*RZ2 = n3) and the column batch widths TC (A/C) and CB
-// (B) at compile time; 0 means "taken from the LocalPlan at run time". The
-// compile-time forms get constant index arithmetic and register allocation
-// sized for their own radices; the all-zero form serves any supported box.
+// Template parameters of A and C fix the radix pairs of the plane (RX1*RX2 = n1, RY1*RY2 = n2) and the
+// column batch width TC at compile time; 0 means "taken from the LocalPlan at run time". The
+// compile-time forms get constant index arithmetic and register allocation sized for their own
+// radices; the all-zero form serves any supported box. B has a compiled form per line length and
+// two run-time forms.
 #pragma once
 #include <algorithm>
 
@@ -15,19 +15,15 @@ namespace kern {
 
 constexpr int kThreadsPlanes = 256;
 constexpr int kThreadsCols = 256;
-// Threads of a CTA of a two-pass (four-step) transform stage: one per line of the larger pass
-// when that is 192 or 384 lines (96- and 144-point lines in 32- or 16-column tiles), so that
-// no pass leaves part of the CTA idle before the barrier; else 256.
-constexpr int pass_threads(int lines_a, int lines_b) {
-  return (lines_a > lines_b ? lines_a : lines_b) == 384 ? 384
-         : (lines_a > lines_b ? lines_a : lines_b) == 192 ? 192 : 256;
-}
-// CTAs per SM asked of the register allocator: two CTAs of 384 threads fit in 80 registers.
-constexpr int pass_min_blocks(int nt) { return nt == 384 ? 2 : 1; }
+// CTAs per SM asked of the register allocator: two CTAs of 320 threads or more (FP64 planes below), as many
+// as two of 384 in 80 registers.
+constexpr int pass_min_blocks(int nt) { return nt >= 320 ? 2 : 1; }
 // Kernels A and C: FP64 planes of 128 points or more take over 200 KB of shared memory (one CTA
-// per SM whatever the registers), so they get no register cap.
+// per SM whatever the registers), so they get no register cap. The run-time form (n1 = 0) would take
+// the registers of its largest radix, one CTA of 256 threads per SM in FP64: it is held to two (FP32:
+// three), at the price of a few spills in radix 16.
 template <typename T> constexpr int plane_min_blocks(int nt, int n1) {
-  return sizeof(T) == 8 && n1 >= 128 ? 1 : pass_min_blocks(nt);
+  return n1 == 0 ? (sizeof(T) == 8 ? 2 : 3) : sizeof(T) == 8 && n1 >= 128 ? 1 : pass_min_blocks(nt);
 }
 
 template <typename T> __device__ __forceinline__ C2<T> czero() { return mk<T>(T(0), T(0)); }
@@ -35,7 +31,9 @@ template <typename T> __device__ __forceinline__ C2<T> czero() { return mk<T>(T(
 // ---------------------------------------------------------------------------
 // A: scatter + inverse x + inverse y, one CTA per (band, kept z-plane)
 // ---------------------------------------------------------------------------
-template <typename T, int RX1, int RX2, int RY1, int RY2, int TC, int NT = kThreadsPlanes>
+// PR: the kept x and y indices lie in the outer quarters of their lines (in_quarters below), so that
+// the first pass of each transform reads and multiplies those points alone.
+template <typename T, int RX1, int RX2, int RY1, int RY2, int TC, bool PR, int NT = kThreadsPlanes>
 __global__ void __launch_bounds__(NT, plane_min_blocks<T>(NT, RX1 * RX2))
 k_inv_xy(LocalPlan p, int band0, const C2<double>* __restrict__ psi, long long ldpsi,
          const int* __restrict__ plane_start, const int* __restrict__ pw_idx,
@@ -80,7 +78,16 @@ k_inv_xy(LocalPlan p, int band0, const C2<double>* __restrict__ psi, long long l
   }
   for (int i = tid; i < n1; i += nt) sx[i] = twx[i];
   for (int i = tid; i < n2; i += nt) sy[i] = twy[i];
-  for (int i = tid; i < ny * rowp; i += nt) R[i] = czero<T>();
+  if constexpr (PR) {
+    // the points that pass 1 reads: the outer quarters of every row
+    const int half = quarter(r1x) * r2x, per = 2 * half;
+    for (int i = tid; i < ny * per; i += nt) {
+      const int row = i / per, x = i - row * per;
+      R[row * rowp + (x < half ? x : n1 - per + x)] = czero<T>();
+    }
+  } else {
+    for (int i = tid; i < ny * rowp; i += nt) R[i] = czero<T>();
+  }
   __syncthreads();
 #pragma unroll
   for (int j = 0; j < kPre; ++j)
@@ -99,10 +106,12 @@ k_inv_xy(LocalPlan p, int band0, const C2<double>* __restrict__ psi, long long l
     C2<T>* line = R + (size_t)row * rowp + n2i;
     with_radix<RX1>(r1x, [&](auto rc_) {
       constexpr int RR = decltype(rc_)::value;
+      constexpr unsigned M = PR ? quarter_bits(RR) : (1u << RR) - 1;
       C2<T> v[RR];
 #pragma unroll
-      for (int a = 0; a < RR; ++a) v[a] = line[r2x * a];
-      DFT<RR, +1, T>::run(v);
+      for (int a = 0; a < RR; ++a)
+        if ((M >> a) & 1) v[a] = line[r2x * a];
+      DFTM<M, RR, +1, T>::run(v);
 #pragma unroll
       for (int a = 0; a < RR; ++a) line[r2x * a] = a == 0 ? v[0] : cmulc<T>(v[a], sx[n2i * a]);
     });
@@ -124,7 +133,10 @@ k_inv_xy(LocalPlan p, int band0, const C2<double>* __restrict__ psi, long long l
   }
   __syncthreads();
 
-  // inverse y on every column, in batches of tc storage positions
+  // inverse y on every column, in batches of tc storage positions. The slab keeps the x storage order
+  // of pass 2 (slab_x): a warp stores 32 neighbouring columns of a row in 512 contiguous bytes. Stored in
+  // x order its 32 pieces of 16 bytes fell r1x columns apart, and the stores took two thirds of the
+  // L1 data path that bounds this kernel.
   C2<T>* Wp = W + ((size_t)b * p.nz + zi) * (size_t)p.plane;
   for (int pb = 0; pb < n1; pb += tc) {
     const int ncol = min(tc, n1 - pb);
@@ -134,13 +146,24 @@ k_inv_xy(LocalPlan p, int band0, const C2<double>* __restrict__ psi, long long l
         with_radix<RY1>(r1y, [&](auto rc_) {
           constexpr int RR = decltype(rc_)::value;
           C2<T> v[RR];
+          if constexpr (PR) {
+            constexpr int Q = quarter(RR);
+            const C2<T>* lo = R + (size_t)n2i * rowp + pb + pl;       // row of y <= kd2
+            const C2<T>* hi = lo - (ptrdiff_t)(n2 - ny) * rowp;       // row of y >= n2 - kd2
 #pragma unroll
-          for (int a = 0; a < RR; ++a) {
-            const int y = r2y * a + n2i;
-            const int yi = idx_to_kept(y, p.kd2, n2, ny);
-            v[a] = yi >= 0 ? R[(size_t)yi * rowp + pb + pl] : czero<T>();
+            for (int a = 0; a < Q; ++a) v[a] = r2y * a + n2i <= p.kd2 ? lo[(size_t)(r2y * a) * rowp] : czero<T>();
+#pragma unroll
+            for (int a = RR - Q; a < RR; ++a)
+              v[a] = r2y * a + n2i >= n2 - p.kd2 ? hi[(size_t)(r2y * a) * rowp] : czero<T>();
+            DFTM<quarter_bits(RR), RR, +1, T>::run(v);
+          } else {
+#pragma unroll
+            for (int a = 0; a < RR; ++a) {
+              const int yi = idx_to_kept(r2y * a + n2i, p.kd2, n2, ny);
+              v[a] = yi >= 0 ? R[(size_t)yi * rowp + pb + pl] : czero<T>();
+            }
+            DFT<RR, +1, T>::run(v);
           }
-          DFT<RR, +1, T>::run(v);
 #pragma unroll
           for (int a = 0; a < RR; ++a)
             Tb[(size_t)(r2y * a + n2i) * tc + pl] = a == 0 ? v[0] : cmulc<T>(v[a], sy[n2i * a]);
@@ -151,9 +174,6 @@ k_inv_xy(LocalPlan p, int band0, const C2<double>* __restrict__ psi, long long l
     for (int it = tid; it < tc * r1y; it += nt) {
       const int pl = it % tc, k1 = it / tc;
       if (pl < ncol) {
-        const int pp = pb + pl;
-        const int xk1 = pp / r2x, xk2 = pp - xk1 * r2x;
-        const int x = xk1 + r1x * xk2;
         with_radix<RY2>(r2y, [&](auto rc_) {
           constexpr int RR = decltype(rc_)::value;
           C2<T> v[RR];
@@ -161,7 +181,7 @@ k_inv_xy(LocalPlan p, int band0, const C2<double>* __restrict__ psi, long long l
           for (int a = 0; a < RR; ++a) v[a] = Tb[(size_t)(r2y * k1 + a) * tc + pl];
           DFT<RR, +1, T>::run(v);
 #pragma unroll
-          for (int a = 0; a < RR; ++a) Wp[(size_t)(k1 + r1y * a) * n1 + x] = v[a];
+          for (int a = 0; a < RR; ++a) Wp[(size_t)(k1 + r1y * a) * n1 + pb + pl] = v[a];
         });
       }
     }
@@ -172,13 +192,11 @@ k_inv_xy(LocalPlan p, int band0, const C2<double>* __restrict__ psi, long long l
 // ---------------------------------------------------------------------------
 // B: inverse z, V(r)/N, forward z, one CTA per (band, CB xy-columns)
 // ---------------------------------------------------------------------------
-template <typename T, int RZ1, int RZ2, int CB>
+template <typename T>
 __global__ void __launch_bounds__(kThreadsCols, 1)
 k_z_vloc(LocalPlan p, const T* __restrict__ vr, const C2<T>* __restrict__ twz, C2<T>* __restrict__ W) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int cb = CB ? CB : p.cb;
-  const int r1 = RZ1 ? RZ1 : p.dz.r1, r2 = RZ2 ? RZ2 : p.dz.r2;
-  const int n3 = RZ1 ? RZ1 * RZ2 : p.n3;
+  const int cb = p.cb, r1 = p.dz.r1, r2 = p.dz.r2, n3 = p.n3;
   C2<T>* Cs = reinterpret_cast<C2<T>*>(smem_raw);
   C2<T>* sz = Cs + (size_t)n3 * cb;
   const long long c0 = (long long)blockIdx.x * cb;
@@ -197,7 +215,7 @@ k_z_vloc(LocalPlan p, const T* __restrict__ vr, const C2<T>* __restrict__ twz, C
   for (int it = tid; it < cb * r2; it += nt) {
     const int cl = it % cb, n2i = it / cb;
     if (cl < ncol) {
-      with_radix<RZ1>(r1, [&](auto rc_) {
+      with_radix<0>(r1, [&](auto rc_) {
         constexpr int RR = decltype(rc_)::value;
         C2<T> v[RR];
 #pragma unroll
@@ -217,12 +235,13 @@ k_z_vloc(LocalPlan p, const T* __restrict__ vr, const C2<T>* __restrict__ twz, C
   for (int it = tid; it < cb * r1; it += nt) {
     const int cl = it % cb, k1 = it / cb;
     if (cl < ncol) {
-      with_radix<RZ2>(r2, [&](auto rc_) {
+      with_radix<0>(r2, [&](auto rc_) {
         constexpr int RR = decltype(rc_)::value;
         C2<T> v[RR];
         T vz[RR];
 #pragma unroll
-        for (int a = 0; a < RR; ++a) vz[a] = vr[(size_t)(k1 + r1 * a) * p.plane + c0 + cl];
+        const long long vc = slab_column(p, c0 + cl);
+        for (int a = 0; a < RR; ++a) vz[a] = vr[(size_t)(k1 + r1 * a) * p.plane + vc];
 #pragma unroll
         for (int a = 0; a < RR; ++a) v[a] = Cs[(size_t)(r2 * k1 + a) * cb + cl];
         DFT<RR, +1, T>::run(v);
@@ -240,7 +259,7 @@ k_z_vloc(LocalPlan p, const T* __restrict__ vr, const C2<T>* __restrict__ twz, C
   for (int it = tid; it < cb * r2; it += nt) {
     const int cl = it % cb, m2 = it / cb;
     if (cl < ncol) {
-      with_radix<RZ1>(r1, [&](auto rc_) {
+      with_radix<0>(r1, [&](auto rc_) {
         constexpr int RR = decltype(rc_)::value;
         C2<T> v[RR];
 #pragma unroll
@@ -276,38 +295,26 @@ __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commi
 template <int N> __device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N)); }
 
 // shared memory of k_z_vloc_pipe: work columns, two staging buffers of kept planes, twiddles, V tile
-template <typename T> inline size_t smem_columns_pipe(const LocalPlan& p, int cb, int nstage = 2) {
-  return smem_columns_pipe_bytes(sizeof(C2<T>), p, cb, nstage);
+template <typename T> inline size_t smem_columns_pipe(const LocalPlan& p, int cb) {
+  return smem_columns_pipe_bytes(sizeof(C2<T>), p, cb);
 }
 
-// NSTAGE: kept-plane staging buffers (2: band b+1 streams in during band b; 1: it streams in
-// during the second and third pass of band b, which frees shared memory for a third CTA per SM).
-// MINB: CTAs per SM asked of the register allocator (0: the pass-size default).
-// TWREG: each thread keeps the z-twiddles of its own line in registers; it needs RZ1 == RZ2 and
-// NT == CB * RZ1, so that every thread owns the same line index in all three passes.
-// VG: V(r)/N read from global memory (L2) in the middle pass instead of a shared-memory tile.
-template <typename T, int RZ1, int RZ2, int CB, int NT = kThreadsCols, int NSTAGE = 2, int MINB = 0,
-          bool TWREG = false, bool VG = false>
-__global__ void __launch_bounds__(NT, MINB ? MINB : pass_min_blocks(NT))
+template <typename T>
+__global__ void __launch_bounds__(kThreadsCols, 1)
 k_z_vloc_pipe(LocalPlan p, int nbc, int bands_per_group, const T* __restrict__ vr, const C2<T>* __restrict__ twz,
               C2<T>* __restrict__ W) {
-  static_assert(NSTAGE == 1 || NSTAGE == 2, "one or two staging buffers");
-  static_assert(!TWREG || (RZ1 == RZ2 && RZ1 > 0 && CB > 0 && NT == CB * RZ1), "register twiddles need one line per thread");
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  const int cb = CB ? CB : p.cb;
-  const int r1 = RZ1 ? RZ1 : p.dz.r1, r2 = RZ2 ? RZ2 : p.dz.r2;
-  const int n3 = RZ1 ? RZ1 * RZ2 : p.n3;
-  const int nz = p.nz;
+  const int cb = p.cb, r1 = p.dz.r1, r2 = p.dz.r2, n3 = p.n3, nz = p.nz;
   C2<T>* Cs = reinterpret_cast<C2<T>*>(smem_raw);
   C2<T>* Ws = Cs + (size_t)n3 * cb;
-  C2<T>* sz = Ws + NSTAGE * (size_t)nz * cb;
+  C2<T>* sz = Ws + 2 * (size_t)nz * cb;
   T* Vs = reinterpret_cast<T*>(sz + n3);
   const long long c0 = (long long)blockIdx.x * cb;
   const int ncol = (int)min((long long)cb, p.plane - c0);
   const int b_lo = blockIdx.y * bands_per_group;
   const int b_hi = min(nbc, b_lo + bands_per_group);
   if (b_lo >= b_hi) return;
-  const int tid = threadIdx.x, nt = NT;     // every launch uses NT threads
+  const int tid = threadIdx.x, nt = kThreadsCols;
 
   auto stage = [&](int b, int buf) {
     const C2<T>* Wb = W + (size_t)b * nz * (size_t)p.plane + c0;
@@ -318,107 +325,60 @@ k_z_vloc_pipe(LocalPlan p, int nbc, int bands_per_group, const T* __restrict__ v
     }
   };
   for (int i = tid; i < n3; i += nt) sz[i] = twz[i];
-  if (!VG) {
-    for (int it = tid; it < cb * n3; it += nt) {
-      const int cl = it % cb, z = it / cb;
-      if (cl < ncol) cp_async_bytes(Vs + (size_t)z * cb + cl, vr + (size_t)z * p.plane + c0 + cl, (int)sizeof(T));
-    }
+  for (int it = tid; it < cb * n3; it += nt) {
+    const int cl = it % cb, z = it / cb;
+    if (cl < ncol)
+      cp_async_bytes(Vs + (size_t)z * cb + cl, vr + (size_t)z * p.plane + slab_column(p, c0 + cl), (int)sizeof(T));
   }
   stage(b_lo, 0);
   cp_async_commit();
-  if (NSTAGE == 2) {
-    if (b_lo + 1 < b_hi) stage(b_lo + 1, 1);
-    cp_async_commit();
-  }
-  // register twiddles: the thread's line index is tid / CB in every pass (n2i of pass 1, k1 of
-  // pass 2); W^(j a) for a = 1 .. R-1 (read once the twiddle table has been written)
-  C2<T> twr[TWREG ? RZ1 : 1];
-  bool tw_loaded = !TWREG;
-  // one pass-1 / pass-3 line per thread (line index j = tid / CB in both): the kept-plane index
-  // of each of its points z = RZ2 a + j, fixed for all bands, is computed once (FP32: the FP64
-  // form has no registers to spare for it under its 3-CTA bound)
-  constexpr bool kOneLine = sizeof(T) == 4 && CB > 0 && RZ1 > 0 && RZ2 > 0 && NT == CB * RZ2;
-  int zk[kOneLine ? RZ1 : 1];
-  if constexpr (kOneLine) {
-#pragma unroll
-    for (int a = 0; a < RZ1; ++a) zk[a] = idx_to_kept(RZ2 * a + tid / CB, p.kd3, n3, nz);
-  }
+  if (b_lo + 1 < b_hi) stage(b_lo + 1, 1);
+  cp_async_commit();
 
   for (int b = b_lo; b < b_hi; ++b) {
-    const int buf = NSTAGE == 2 ? (b - b_lo) & 1 : 0;
-    if (NSTAGE == 2)
-      cp_async_wait<1>();     // every group but the newest (band b+1) has landed
-    else
-      cp_async_wait<0>();     // band b has landed
+    const int buf = (b - b_lo) & 1;
+    cp_async_wait<1>();     // every group but the newest (band b+1) has landed
     __syncthreads();
-    if (TWREG && !tw_loaded) {
-      const int j = tid / (CB ? CB : 1);
-#pragma unroll
-      for (int a = 0; a < (TWREG ? RZ1 : 1); ++a) twr[a] = sz[(j * a) % n3];
-      tw_loaded = true;
-    }
     const C2<T>* Wsb = Ws + (size_t)buf * nz * cb;
     // inverse pass 1 straight from the staged kept planes
     for (int it = tid; it < cb * r2; it += nt) {
       const int cl = it % cb, n2i = it / cb;
       if (cl < ncol) {
-        with_radix<RZ1>(r1, [&](auto rc_) {
+        with_radix<0>(r1, [&](auto rc_) {
           constexpr int RR = decltype(rc_)::value;
           C2<T> v[RR];
 #pragma unroll
           for (int a = 0; a < RR; ++a) {
-            int zi;
-            if constexpr (kOneLine)
-              zi = zk[a];
-            else
-              zi = idx_to_kept(r2 * a + n2i, p.kd3, n3, nz);
+            const int zi = idx_to_kept(r2 * a + n2i, p.kd3, n3, nz);
             v[a] = zi >= 0 ? Wsb[(size_t)zi * cb + cl] : czero<T>();
           }
           DFT<RR, +1, T>::run(v);
 #pragma unroll
-          for (int a = 0; a < RR; ++a) {
-            if constexpr (TWREG)
-              Cs[(size_t)(r2 * a + n2i) * cb + cl] = a == 0 ? v[0] : cmulc<T>(v[a], twr[a]);
-            else
-              Cs[(size_t)(r2 * a + n2i) * cb + cl] = a == 0 ? v[0] : cmulc<T>(v[a], sz[n2i * a]);
-          }
+          for (int a = 0; a < RR; ++a)
+            Cs[(size_t)(r2 * a + n2i) * cb + cl] = a == 0 ? v[0] : cmulc<T>(v[a], sz[n2i * a]);
         });
       }
     }
     __syncthreads();
-    // the staging buffer of band b is free: prefetch band b+2 (two buffers) or b+1 (one) into it
-    if (b + NSTAGE < b_hi) stage(b + NSTAGE, buf);
+    // the staging buffer of band b is free: prefetch band b+2 into it
+    if (b + 2 < b_hi) stage(b + 2, buf);
     cp_async_commit();
     // inverse pass 2 -> V/N -> forward pass 1, in registers
     for (int it = tid; it < cb * r1; it += nt) {
       const int cl = it % cb, k1 = it / cb;
       if (cl < ncol) {
-        with_radix<RZ2>(r2, [&](auto rc_) {
+        with_radix<0>(r2, [&](auto rc_) {
           constexpr int RR = decltype(rc_)::value;
           C2<T> v[RR];
-          T vz[VG ? RR : 1];
-          if constexpr (VG) {
-#pragma unroll
-            for (int a = 0; a < RR; ++a) vz[a] = __ldg(vr + (size_t)(k1 + r1 * a) * p.plane + c0 + cl);
-          }
 #pragma unroll
           for (int a = 0; a < RR; ++a) v[a] = Cs[(size_t)(r2 * k1 + a) * cb + cl];
           DFT<RR, +1, T>::run(v);
 #pragma unroll
-          for (int a = 0; a < RR; ++a) {
-            if constexpr (VG)
-              v[a] = scal<T>(v[a], vz[a]);
-            else
-              v[a] = scal<T>(v[a], Vs[(size_t)(k1 + r1 * a) * cb + cl]);
-          }
+          for (int a = 0; a < RR; ++a) v[a] = scal<T>(v[a], Vs[(size_t)(k1 + r1 * a) * cb + cl]);
           DFT<RR, -1, T>::run(v);
 #pragma unroll
-          for (int a = 0; a < RR; ++a) {
-            if constexpr (TWREG)
-              Cs[(size_t)(r2 * k1 + a) * cb + cl] = a == 0 ? v[0] : cmul<T>(v[a], twr[a]);
-            else
-              Cs[(size_t)(r2 * k1 + a) * cb + cl] = a == 0 ? v[0] : cmul<T>(v[a], sz[k1 * a]);
-          }
+          for (int a = 0; a < RR; ++a)
+            Cs[(size_t)(r2 * k1 + a) * cb + cl] = a == 0 ? v[0] : cmul<T>(v[a], sz[k1 * a]);
         });
       }
     }
@@ -428,7 +388,7 @@ k_z_vloc_pipe(LocalPlan p, int nbc, int bands_per_group, const T* __restrict__ v
     for (int it = tid; it < cb * r2; it += nt) {
       const int cl = it % cb, m2 = it / cb;
       if (cl < ncol) {
-        with_radix<RZ1>(r1, [&](auto rc_) {
+        with_radix<0>(r1, [&](auto rc_) {
           constexpr int RR = decltype(rc_)::value;
           C2<T> v[RR];
 #pragma unroll
@@ -436,11 +396,7 @@ k_z_vloc_pipe(LocalPlan p, int nbc, int bands_per_group, const T* __restrict__ v
           DFT<RR, -1, T>::run(v);
 #pragma unroll
           for (int a = 0; a < RR; ++a) {
-            int zi;
-            if constexpr (kOneLine)
-              zi = zk[a];
-            else
-              zi = idx_to_kept(m2 + r2 * a, p.kd3, n3, nz);
+            const int zi = idx_to_kept(m2 + r2 * a, p.kd3, n3, nz);
             if (zi >= 0) Wb[(size_t)zi * p.plane + cl] = v[a];
           }
         });
@@ -451,9 +407,109 @@ k_z_vloc_pipe(LocalPlan p, int nbc, int bands_per_group, const T* __restrict__ v
 }
 
 // ---------------------------------------------------------------------------
+// B (register form): one CTA per (CB xy-columns, band group) with one thread per line of the outer
+// passes, for kept planes in the outer quarters of the z lines (in_quarters). A thread owns the same
+// column and line index j in the inverse's first and the forward's last pass, so it reads its kept
+// points of the slab straight into registers (those of band b + 1 while band b is transformed: no
+// staging buffers), starts from the nonzero half of the line (DFTM), keeps only the kept outputs of the
+// last pass, and needs two barriers per band: what pass 1 of band b + 1 overwrites in shared memory the
+// same thread has read in the last pass of band b.
+// ---------------------------------------------------------------------------
+template <typename T, int R1, int R2, int CB> constexpr int z_min_blocks() {
+  return std::max(1, 65536 / (CB * R2 * (sizeof(T) == 8 ? 112 : 64)));
+}
+template <typename T, int R1, int R2, int CB>
+__global__ void __launch_bounds__(CB * R2, (z_min_blocks<T, R1, R2, CB>()))
+k_z_band(LocalPlan p, int nbc, int per, const T* __restrict__ vr, const C2<T>* __restrict__ twz, C2<T>* __restrict__ W) {
+  constexpr int N3 = R1 * R2, NT = CB * R2, Q = quarter(R1);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C2<T>* Cs = reinterpret_cast<C2<T>*>(smem_raw);
+  C2<T>* sz = Cs + N3 * CB;
+  T* Vs = reinterpret_cast<T*>(sz + N3);
+  const int tid = threadIdx.x, cl = tid % CB, j = tid / CB;
+  const size_t pl = (size_t)p.plane;
+  const long long col = (long long)blockIdx.x * CB + cl;
+  const bool ok = col < p.plane;
+  const int b_lo = blockIdx.y * per, b_hi = min(nbc, b_lo + per);
+  if (b_lo >= b_hi) return;
+  const int kd = p.kd3, skip = N3 - p.nz;
+  C2<T>* Wb = W + (size_t)b_lo * p.nz * pl + col;
+  const size_t band = (size_t)p.nz * pl;
+
+  C2<T> nx[2 * Q];       // kept points z = R2 a + j, a < Q and a >= R1 - Q, of the next band
+  auto load = [&](const C2<T>* w) {
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const int z = R2 * q + j;
+      nx[q] = ok && z <= kd ? w[z * pl] : czero<T>();
+    }
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const int z = R2 * (R1 - Q + q) + j;
+      nx[Q + q] = ok && z >= N3 - kd ? w[(z - skip) * pl] : czero<T>();
+    }
+  };
+  load(Wb);
+  for (int i = tid; i < N3; i += NT) sz[i] = twz[i];
+  {
+    // all of the thread's V values in flight at once
+    const T* vc = vr + (ok ? slab_column(p, col) : 0);
+    T v[R1];
+#pragma unroll
+    for (int a = 0; a < R1; ++a) v[a] = ok ? vc[(R2 * a + j) * pl] : T(0);
+#pragma unroll
+    for (int a = 0; a < R1; ++a) Vs[(R2 * a + j) * CB + cl] = v[a];
+  }
+  __syncthreads();
+
+  for (int b = b_lo; b < b_hi; ++b, Wb += band) {
+    {
+      C2<T> v[R1];
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        v[q] = nx[q];
+        v[R1 - Q + q] = nx[Q + q];
+      }
+      DFTM<quarter_bits(R1), R1, +1, T>::run(v);
+#pragma unroll
+      for (int a = 0; a < R1; ++a) Cs[(R2 * a + j) * CB + cl] = a == 0 ? v[0] : cmulc<T>(v[a], sz[j * a]);
+    }
+    if (b + 1 < b_hi) load(Wb + band);
+    __syncthreads();
+    if (R1 == R2 || j < R1) {
+      C2<T> v[R2];
+#pragma unroll
+      for (int a = 0; a < R2; ++a) v[a] = Cs[(R2 * j + a) * CB + cl];
+      DFT<R2, +1, T>::run(v);
+#pragma unroll
+      for (int a = 0; a < R2; ++a) v[a] = scal<T>(v[a], Vs[(j + R1 * a) * CB + cl]);
+      DFT<R2, -1, T>::run(v);
+#pragma unroll
+      for (int a = 0; a < R2; ++a) Cs[(R2 * j + a) * CB + cl] = a == 0 ? v[0] : cmul<T>(v[a], sz[j * a]);
+    }
+    __syncthreads();
+    {
+      C2<T> v[R1];
+#pragma unroll
+      for (int a = 0; a < R1; ++a) v[a] = Cs[(R2 * a + j) * CB + cl];
+      DFT<R1, -1, T>::run(v);
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const int z = R2 * q + j, zh = R2 * (R1 - Q + q) + j;
+        if (ok && z <= kd) Wb[z * pl] = v[q];
+        if (ok && zh >= N3 - kd) Wb[(zh - skip) * pl] = v[R1 - Q + q];
+      }
+    }
+  }
+}
+template <typename T, int R1, int R2, int CB> constexpr size_t smem_z_band() {
+  return (size_t)R1 * R2 * (CB * (sizeof(C2<T>) + sizeof(T)) + sizeof(C2<T>));
+}
+
+// ---------------------------------------------------------------------------
 // C: forward y + forward x + gather + kinetic, one CTA per (band, kept z-plane)
 // ---------------------------------------------------------------------------
-template <typename T, int RX1, int RX2, int RY1, int RY2, int TC, int NT = kThreadsPlanes>
+template <typename T, int RX1, int RX2, int RY1, int RY2, int TC, bool PR, int NT = kThreadsPlanes>
 __global__ void __launch_bounds__(NT, plane_min_blocks<T>(NT, RX1 * RX2))
 k_fwd_xy(LocalPlan p, int band0, const C2<double>* __restrict__ psi, long long ldpsi,
          C2<double>* __restrict__ hpsi, long long ldh, const int* __restrict__ plane_start,
@@ -489,26 +545,26 @@ k_fwd_xy(LocalPlan p, int band0, const C2<double>* __restrict__ psi, long long l
   const int e0 = plane_start[zi], e1 = plane_start[zi + 1];
 
   const C2<T>* Wp = W + ((size_t)b * p.nz + zi) * (size_t)p.plane;
+  if (tid == 0 && p.plane * sizeof(C2<T>) % 16 == 0) {
+    // bring the plane into L2 while the first tiles are transformed
+    const char* w = reinterpret_cast<const char*>(Wp);
+    const size_t bytes = (size_t)p.plane * sizeof(C2<T>);
+    for (size_t o = 0; o < bytes; o += 16384)
+      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;\n" ::"l"(w + o), "r"((unsigned)min((size_t)16384, bytes - o)) : "memory");
+  }
+  __syncthreads();      // the twiddles
+  // Where a large FP64 plane leaves one CTA per SM and every thread has one line per pass, the next
+  // tile's points are loaded while this one is transformed: nothing else hides their latency there
+  // (144 x 144: 4.47 -> 4.28 ms per 480 bands).
+  constexpr bool kAhead = sizeof(T) == 8 && RX1 * RX2 >= 128 && TC * RY2 == NT;
+  C2<T> ahead[kAhead ? RY1 : 1];
+  if constexpr (kAhead) {
+#pragma unroll
+    for (int a = 0; a < RY1; ++a) ahead[a] = Wp[(size_t)(RY2 * a + tid / TC) * n1 + tid % TC];
+  }
   for (int xb = 0; xb < n1; xb += tc) {
     const int ncol = min(tc, n1 - xb);
-    // the tile's columns of every y row, all copies in flight at once
-    for (int it = tid; it < tc * n2; it += nt) {
-      const int xl = it % tc, y = it / tc;
-      if (xl < ncol) cp_async_bytes(Tb + (size_t)y * tc + xl, Wp + (size_t)y * n1 + xb + xl, (int)sizeof(C2<T>));
-    }
-    cp_async_commit();
-    if (sizeof(T) == 8 && xb == 0 && ekpg) {
-      // while the first tile lands: bring the psi values and kinetic terms of the final gather
-      // into L2, so that its dependent loads do not wait on HBM at the end of the CTA (FP64
-      // only: in FP32 the extra registers cost a CTA per SM on 96-point lines)
-      for (int e = e0 + tid; e < e1; e += nt) {
-        const int i = pw_idx[e];
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(ps + i));
-        asm volatile("prefetch.global.L2 [%0];" ::"l"(ekpg + i));
-      }
-    }
-    cp_async_wait<0>();
-    __syncthreads();
+    // pass 1 from the slab (a warp reads neighbouring columns of a row), pass 2 into the kept rows
     for (int it = tid; it < tc * r2y; it += nt) {
       const int xl = it % tc, n2i = it / tc;
       if (xl < ncol) {
@@ -516,12 +572,33 @@ k_fwd_xy(LocalPlan p, int band0, const C2<double>* __restrict__ psi, long long l
           constexpr int RR = decltype(rc_)::value;
           C2<T> v[RR];
 #pragma unroll
-          for (int a = 0; a < RR; ++a) v[a] = Tb[(size_t)(r2y * a + n2i) * tc + xl];
+          for (int a = 0; a < RR; ++a) {
+            if constexpr (kAhead)
+              v[a] = ahead[a];
+            else
+              v[a] = Wp[(size_t)(r2y * a + n2i) * n1 + xb + xl];
+          }
           DFT<RR, -1, T>::run(v);
 #pragma unroll
           for (int a = 0; a < RR; ++a)
             Tb[(size_t)(r2y * a + n2i) * tc + xl] = a == 0 ? v[0] : cmul<T>(v[a], sy[n2i * a]);
+          if constexpr (kAhead) {
+            if (xb + tc + xl < n1) {
+#pragma unroll
+              for (int a = 0; a < RR; ++a) ahead[a] = Wp[(size_t)(r2y * a + n2i) * n1 + xb + tc + xl];
+            }
+          }
         });
+      }
+    }
+    if (sizeof(T) == 8 && xb == 0 && ekpg) {
+      // bring the psi values and kinetic terms of the final gather into L2, so that its dependent
+      // loads do not wait on HBM at the end of the CTA (FP64 only: in FP32 the extra registers cost a
+      // CTA per SM on 96-point lines)
+      for (int e = e0 + tid; e < e1; e += nt) {
+        const int i = pw_idx[e];
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(ps + i));
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(ekpg + i));
       }
     }
     __syncthreads();
@@ -534,10 +611,22 @@ k_fwd_xy(LocalPlan p, int band0, const C2<double>* __restrict__ psi, long long l
 #pragma unroll
           for (int a = 0; a < RR; ++a) v[a] = Tb[(size_t)(r2y * k1 + a) * tc + xl];
           DFT<RR, -1, T>::run(v);
+          if constexpr (PR) {
+            constexpr int Q = quarter(RR);
+            C2<T>* lo = R + (size_t)k1 * rowp + xb + xl;
+            C2<T>* hi = lo - (ptrdiff_t)(n2 - ny) * rowp;
 #pragma unroll
-          for (int a = 0; a < RR; ++a) {
-            const int yi = idx_to_kept(k1 + r1y * a, p.kd2, n2, ny);
-            if (yi >= 0) R[(size_t)yi * rowp + xb + xl] = v[a];
+            for (int a = 0; a < Q; ++a)
+              if (k1 + r1y * a <= p.kd2) lo[(size_t)(r1y * a) * rowp] = v[a];
+#pragma unroll
+            for (int a = RR - Q; a < RR; ++a)
+              if (k1 + r1y * a >= n2 - p.kd2) hi[(size_t)(r1y * a) * rowp] = v[a];
+          } else {
+#pragma unroll
+            for (int a = 0; a < RR; ++a) {
+              const int yi = idx_to_kept(k1 + r1y * a, p.kd2, n2, ny);
+              if (yi >= 0) R[(size_t)yi * rowp + xb + xl] = v[a];
+            }
           }
         });
       }
@@ -545,43 +634,59 @@ k_fwd_xy(LocalPlan p, int band0, const C2<double>* __restrict__ psi, long long l
     __syncthreads();
   }
 
-  // forward x on the kept rows (row index fastest across lanes)
+  // forward x on the kept rows (row index fastest across lanes). The points lie in the slab's storage
+  // order: slot(x) is where natural index x is (run-time radices: from a table in the tile buffer, which
+  // is free by now and at least n1 shorts long: two rows of 32 columns, or more rows).
+  unsigned short* sslot = reinterpret_cast<unsigned short*>(Tb);
+  if constexpr (RX1 == 0) {
+    for (int i = tid; i < n1; i += nt) sslot[i] = (unsigned short)slab_slot(i, r1x, r2x);
+    __syncthreads();
+  }
+  auto slot = [&](int x) { return RX1 ? slab_slot(x, r1x, r2x) : (int)sslot[x]; };
   for (int it = tid; it < ny * r2x; it += nt) {
     const int row = it % ny, n2i = it / ny;
-    C2<T>* line = R + (size_t)row * rowp + n2i;
+    C2<T>* line = R + (size_t)row * rowp;
     with_radix<RX1>(r1x, [&](auto rc_) {
       constexpr int RR = decltype(rc_)::value;
       C2<T> v[RR];
+      int at[RR];
 #pragma unroll
-      for (int a = 0; a < RR; ++a) v[a] = line[r2x * a];
+      for (int a = 0; a < RR; ++a) {
+        at[a] = RX1 && RX1 == RX2 ? RX1 * n2i + a : slot(r2x * a + n2i);
+        v[a] = line[at[a]];
+      }
       DFT<RR, -1, T>::run(v);
 #pragma unroll
-      for (int a = 0; a < RR; ++a) line[r2x * a] = a == 0 ? v[0] : cmul<T>(v[a], sx[n2i * a]);
+      for (int a = 0; a < RR; ++a) line[at[a]] = a == 0 ? v[0] : cmul<T>(v[a], sx[n2i * a]);
     });
   }
   __syncthreads();
   for (int it = tid; it < ny * r1x; it += nt) {
     const int row = it % ny, k1 = it / ny;
-    C2<T>* line = R + (size_t)row * rowp + r2x * k1;
+    C2<T>* line = R + (size_t)row * rowp;
     with_radix<RX2>(r2x, [&](auto rc_) {
       constexpr int RR = decltype(rc_)::value;
+      constexpr unsigned M = PR ? quarter_bits(RR) : (1u << RR) - 1;
       C2<T> v[RR];
+      int at[RR];
 #pragma unroll
-      for (int a = 0; a < RR; ++a) v[a] = line[a];
+      for (int a = 0; a < RR; ++a) {
+        at[a] = RX1 && RX1 == RX2 ? RX1 * a + k1 : slot(r2x * k1 + a);
+        v[a] = line[at[a]];
+      }
       DFT<RR, -1, T>::run(v);
 #pragma unroll
-      for (int a = 0; a < RR; ++a) line[a] = v[a];
+      for (int a = 0; a < RR; ++a)
+        if ((M >> a) & 1) line[at[a]] = v[a];       // frequency k1 + r1x a
     });
   }
   __syncthreads();
 
-  // gather the sphere (permuted x storage) and add the kinetic diagonal
+  // gather the sphere and add the kinetic diagonal
   for (int e = e0 + tid; e < e1; e += nt) {
     const int pos = pw_pos[e];
-    const int x = pos & 0xffff, yi = pos >> 16;
-    const int q = x / r1x;
-    const int pp = r2x * (x - q * r1x) + q;
-    const C2<T> v = R[(size_t)yi * rowp + pp];
+    const int x = pos & 0xffff, q = x / r1x;
+    const C2<T> v = R[(size_t)(pos >> 16) * rowp + slot(r2x * (x - q * r1x) + q)];
     const int i = pw_idx[e];
     C2<double> out = mk<double>(double(v.x), double(v.y));
     if (ekpg) {
@@ -599,86 +704,75 @@ k_fwd_xy(LocalPlan p, int band0, const C2<double>* __restrict__ psi, long long l
   }
 }
 
-// Launch A, B, C for one band chunk with one compile-time configuration.
-template <typename T, int RX1, int RX2, int RY1, int RY2, int RZ1, int RZ2, int TC, int CB>
-cudaError_t launch_impl(const LocalPlan& p, int nbc, int band0, const C2<double>* psi, long long ldpsi,
-                        C2<double>* hpsi, long long ldh, const int* plane_start, const int* pw_idx,
-                        const int* pw_pos, const double* ekpg, const T* vr, const C2<T>* twx, const C2<T>* twy,
-                        const C2<T>* twz, C2<T>* W, cudaStream_t st, cudaEvent_t* ev) {
-  constexpr int NTP = TC && RY1 ? pass_threads(TC * RY2, TC * RY1) : kThreadsPlanes;
-  constexpr int NTZ = CB && RZ1 ? pass_threads(CB * RZ2, CB * RZ1) : kThreadsCols;
-  // C keeps 256 threads where 384 measured slower: FP32 on 96-point lines.
-  constexpr bool c_wide = sizeof(T) == 8 || RY1 * RY2 >= 128;
-  constexpr int NTC = NTP == 384 && c_wide ? 384 : kThreadsPlanes;
-  const size_t sm_pl = smem_planes<T>(p);
-  auto* ka = k_inv_xy<T, RX1, RX2, RY1, RY2, TC, NTP>;
-  auto* kc = k_fwd_xy<T, RX1, RX2, RY1, RY2, TC, NTC>;
-  cudaError_t e;
-  if ((e = smem_limit((const void*)ka, (size_t)sm_pl)) != cudaSuccess) return e;
-  if ((e = smem_limit((const void*)kc, (size_t)sm_pl)) != cudaSuccess) return e;
-  int nsm = 148, dev = 0, smax = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
-  cudaDeviceGetAttribute(&smax, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
-  dim3 gA(p.nz, nbc);
-  if (ev) cudaEventRecord(ev[0], st);
-  ka<<<gA, NTP, sm_pl, st>>>(p, band0, psi, ldpsi, plane_start, pw_idx, pw_pos, twx, twy, W);
-  if (ev) cudaEventRecord(ev[1], st);
-  // kernel B form on boxes whose z split is square (one line per thread in every pass):
-  // CPW_B200_ZB_VARIANT 1 = one staging buffer + 3 CTAs per SM (the default there: on the 144^3
-  // box, 480 bands, FP64 B 8.58 -> 7.17 ms, FP32 5.38 -> 5.32 ms, identical results),
-  // 2 = register twiddles (FP32 6.49 ms), 3 = both, 4 = one staging buffer, V(r)/N from L2 and 4
-  // CTAs per SM, 5 = the same with 3 CTAs; 0 = two staging buffers, twiddles in shared memory (the
-  // only form elsewhere)
-  int zv = 0;
-  if constexpr (RZ1 == RZ2 && RZ1 > 0 && CB > 0 && NTZ == CB * RZ1) {
-    zv = 1;
-    if (const char* v = getenv("CPW_B200_ZB_VARIANT")) zv = std::max(0, std::min(5, atoi(v)));
-  }
-  size_t sm_pipe = smem_columns_pipe<T>(p, p.cb, zv == 1 || zv >= 3 ? 1 : 2);
-  if (zv >= 4) sm_pipe -= sizeof(T) * (size_t)p.n3 * p.cb;     // no V tile
-  const long long tiles = (p.plane + p.cb - 1) / p.cb;
-  if (sm_pipe > (size_t)smax) {
-    // the staged form does not fit: one CTA per (band, column tile)
-    const size_t sm_co = smem_columns<T>(p);
-    auto* kb = k_z_vloc<T, RZ1, RZ2, CB>;
-    if ((e = smem_limit((const void*)kb, (size_t)sm_co)) != cudaSuccess) return e;
-    kb<<<dim3((unsigned)tiles, nbc), kThreadsCols, sm_co, st>>>(p, vr, twz, W);
-  } else {
-    // column tiles x band groups: enough CTAs for two per SM on small boxes
-    const long long per_sm = p.bgroups > 0 ? p.bgroups : 2;
-    long long groups = std::max(1LL, std::min((long long)nbc, (per_sm * nsm + tiles - 1) / tiles));
-    const int per = (int)((nbc + groups - 1) / groups);
-    groups = (nbc + per - 1) / per;
-    auto* kbp = k_z_vloc_pipe<T, RZ1, RZ2, CB, NTZ>;
-    if constexpr (RZ1 == RZ2 && RZ1 > 0 && CB > 0 && NTZ == CB * RZ1) {
-      if (zv == 1) kbp = k_z_vloc_pipe<T, RZ1, RZ2, CB, NTZ, 1, 3, false>;
-      if (zv == 2) kbp = k_z_vloc_pipe<T, RZ1, RZ2, CB, NTZ, 2, 0, true>;
-      if (zv == 3) kbp = k_z_vloc_pipe<T, RZ1, RZ2, CB, NTZ, 1, 3, true>;
-      if (zv == 4) kbp = k_z_vloc_pipe<T, RZ1, RZ2, CB, NTZ, 1, 4, false, true>;
-      if (zv == 5) kbp = k_z_vloc_pipe<T, RZ1, RZ2, CB, NTZ, 1, 3, false, true>;
-    }
-    if ((e = smem_limit((const void*)kbp, (size_t)sm_pipe)) != cudaSuccess)
-      return e;
-    kbp<<<dim3((unsigned)tiles, (unsigned)groups), NTZ, sm_pipe, st>>>(p, nbc, per, vr, twz, W);
-  }
-  if (ev) cudaEventRecord(ev[2], st);
-  kc<<<gA, NTC, sm_pl, st>>>(p, band0, psi, ldpsi, hpsi, ldh, plane_start, pw_idx, pw_pos, ekpg, twx, twy, W);
-  if (ev) cudaEventRecord(ev[3], st);
-  return cudaGetLastError();
+// Threads of kernels A and C: one per line of the larger y pass; C keeps 256 where 384 measured slower
+// (FP32 on 96-point lines: 189 against 176 us for 160 bands).
+template <int RY1, int RY2, int TC> constexpr int threads_a() { return TC && RY1 ? TC * RY2 : kThreadsPlanes; }
+template <typename T, int RY1, int RY2, int TC> constexpr int threads_c() {
+  return sizeof(T) == 4 && RY1 * RY2 == 96 ? kThreadsPlanes : threads_a<RY1, RY2, TC>();
 }
 
 // Launch kernel A alone (scatter + inverse x + inverse y into the slab W).
 template <typename T, int RX1, int RX2, int RY1, int RY2, int TC>
-cudaError_t launch_inv_impl(const LocalPlan& p, int nbc, int band0, const C2<double>* psi, long long ldpsi,
-                            const int* plane_start, const int* pw_idx, const int* pw_pos, const C2<T>* twx,
-                            const C2<T>* twy, C2<T>* W, cudaStream_t st) {
-  constexpr int NTP = TC && RY1 ? pass_threads(TC * RY2, TC * RY1) : kThreadsPlanes;
-  const size_t sm_pl = smem_planes<T>(p);
-  auto* ka = k_inv_xy<T, RX1, RX2, RY1, RY2, TC, NTP>;
-  cudaError_t e = smem_limit((const void*)ka, (size_t)sm_pl);
+cudaError_t launch_a_impl(const LocalPlan& p, int nbc, int band0, const C2<double>* psi, long long ldpsi,
+                          const int* plane_start, const int* pw_idx, const int* pw_pos, const C2<T>* twx,
+                          const C2<T>* twy, C2<T>* W, cudaStream_t st) {
+  constexpr int NT = threads_a<RY1, RY2, TC>();
+  const size_t sm = smem_planes<T>(p);
+  const bool pr = in_quarters(p.kd1, p.dx.r1, p.dx.r2) && in_quarters(p.kd2, p.dy.r1, p.dy.r2);
+  auto* k = pr ? k_inv_xy<T, RX1, RX2, RY1, RY2, TC, true, NT> : k_inv_xy<T, RX1, RX2, RY1, RY2, TC, false, NT>;
+  cudaError_t e = smem_limit((const void*)k, sm);
   if (e != cudaSuccess) return e;
-  ka<<<dim3(p.nz, nbc), NTP, sm_pl, st>>>(p, band0, psi, ldpsi, plane_start, pw_idx, pw_pos, twx, twy, W);
+  k<<<dim3(p.nz, nbc), NT, sm, st>>>(p, band0, psi, ldpsi, plane_start, pw_idx, pw_pos, twx, twy, W);
+  return cudaGetLastError();
+}
+
+// Launch kernel C alone (forward y + forward x from the slab W, gather).
+template <typename T, int RX1, int RX2, int RY1, int RY2, int TC>
+cudaError_t launch_c_impl(const LocalPlan& p, int nbc, int band0, const C2<double>* psi, long long ldpsi,
+                          C2<double>* hpsi, long long ldh, const int* plane_start, const int* pw_idx,
+                          const int* pw_pos, const double* ekpg, const C2<T>* twx, const C2<T>* twy, const C2<T>* W,
+                          cudaStream_t st) {
+  constexpr int NT = threads_c<T, RY1, RY2, TC>();
+  const size_t sm = smem_planes<T>(p);
+  const bool pr = in_quarters(p.kd1, p.dx.r2, p.dx.r1) && in_quarters(p.kd2, p.dy.r2, p.dy.r1);
+  auto* k = pr ? k_fwd_xy<T, RX1, RX2, RY1, RY2, TC, true, NT> : k_fwd_xy<T, RX1, RX2, RY1, RY2, TC, false, NT>;
+  cudaError_t e = smem_limit((const void*)k, sm);
+  if (e != cudaSuccess) return e;
+  k<<<dim3(p.nz, nbc), NT, sm, st>>>(p, band0, psi, ldpsi, hpsi, ldh, plane_start, pw_idx, pw_pos, ekpg, twx, twy, W);
+  return cudaGetLastError();
+}
+
+// Band groups of kernel B: every CTA stages its V tile once (about 0.7 of a band's time) and then takes
+// `per` bands; the split whose busiest SM finishes first. About three CTAs of an SM overlap: fewer take
+// as long as one, more share it. p.bgroups > 0: that many CTAs per SM instead.
+inline int band_groups(const LocalPlan& p, long long tiles, int nbc, int nsm) {
+  if (p.bgroups > 0)
+    return (int)std::max(1LL, std::min((long long)nbc, ((long long)p.bgroups * nsm + tiles - 1) / tiles));
+  int best = 1;
+  double cost = 1e300;
+  for (int g = 1; g <= std::min(nbc, 64); ++g) {
+    const double ctas = (double)((tiles * g + nsm - 1) / nsm);
+    const double c = std::max(1.0, ctas / 3.0) * ((nbc + g - 1) / g + 0.7);
+    if (c < cost * 0.99) {
+      cost = c;
+      best = g;
+    }
+  }
+  return best;
+}
+
+// Launch the register form of kernel B for a z split R1 x R2.
+template <typename T, int R1, int R2>
+cudaError_t launch_z_impl(const LocalPlan& p, int nbc, const T* vr, const C2<T>* twz, C2<T>* W, int nsm,
+                          cudaStream_t st) {
+  constexpr int CB = 16;
+  constexpr size_t sm = smem_z_band<T, R1, R2, CB>();
+  auto* k = k_z_band<T, R1, R2, CB>;
+  cudaError_t e = smem_limit((const void*)k, sm);
+  if (e != cudaSuccess) return e;
+  const long long tiles = (p.plane + CB - 1) / CB;
+  const int g = band_groups(p, tiles, nbc, nsm), per = (nbc + g - 1) / g;
+  k<<<dim3((unsigned)tiles, (unsigned)((nbc + per - 1) / per)), CB * R2, sm, st>>>(p, nbc, per, vr, twz, W);
   return cudaGetLastError();
 }
 
@@ -694,8 +788,16 @@ cudaError_t launch_inv_impl(const LocalPlan& p, int nbc, int band0, const C2<dou
       const T *vr, const C2<T>*twx, const C2<T>*twy, const C2<T>*twz, C2<T>*W, cudaStream_t st,             \
       cudaEvent_t *ev
 
-#define CPWB_INSTANTIATE(T, RX1, RX2, RY1, RY2, RZ1, RZ2, TC, CB)                                        \
-  template cudaError_t kern::launch_impl<T, RX1, RX2, RY1, RY2, RZ1, RZ2, TC, CB>(CPWB_LAUNCH_ARGS(T)); \
-  template cudaError_t kern::launch_inv_impl<T, RX1, RX2, RY1, RY2, TC>(CPWB_INV_ARGS(T));
+#define CPWB_C_ARGS(T)                                                                                       \
+  const LocalPlan &p, int nbc, int band0, const C2<double>*psi, long long ldpsi, C2<double>*hpsi,            \
+      long long ldh, const int *plane_start, const int *pw_idx, const int *pw_pos, const double *ekpg,       \
+      const C2<T>*twx, const C2<T>*twy, const C2<T>*W, cudaStream_t st
+#define CPWB_Z_ARGS(T) const LocalPlan &p, int nbc, const T *vr, const C2<T>*twz, C2<T>*W, int nsm, cudaStream_t st
+
+// kernels A and C for planes r1 r2 x r1 r2, kernel B for z lines of r1 r2 points
+#define CPWB_PLANES(EXTERN, T, R1, R2, TC)                                                           \
+  EXTERN template cudaError_t kern::launch_a_impl<T, R1, R2, R1, R2, TC>(CPWB_INV_ARGS(T));          \
+  EXTERN template cudaError_t kern::launch_c_impl<T, R1, R2, R1, R2, TC>(CPWB_C_ARGS(T));
+#define CPWB_LINES(EXTERN, T, R1, R2) EXTERN template cudaError_t kern::launch_z_impl<T, R1, R2>(CPWB_Z_ARGS(T));
 
 }  // namespace cpwb

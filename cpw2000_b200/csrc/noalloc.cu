@@ -218,9 +218,7 @@ extern "C" int cpw_b200_hk_psi_loc_noalloc(int mtxd, int neig, const void* psi, 
   int smax = 0;
   cudaDeviceGetAttribute(&smax, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
   const size_t es = sizeof(C2<double>);
-  p.tcol = 32;
-  while (p.tcol > 4 && es * ((size_t)p.ny * p.rowp + (size_t)n2 * p.tcol + n1 + n2) > (size_t)smax) p.tcol /= 2;
-  if (es * ((size_t)p.ny * p.rowp + (size_t)n2 * p.tcol + n1 + n2) > (size_t)smax)
+  if (!plane_tile(es, p, (size_t)smax))
     return fail(kUnsupported, "hk_psi_loc_noalloc: plane does not fit in shared memory");
   int smsm = 0;
   cudaDeviceGetAttribute(&smsm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);

@@ -17,7 +17,6 @@
 #include <vector>
 
 #include "context.hpp"
-#include "hkpsi_kernels.cuh"
 
 namespace cpwb {
 
@@ -81,6 +80,7 @@ k_z_spinor(LocalPlan p, int nbc, const T* __restrict__ vu, const T* __restrict__
   for (int it = tid; it < kSpCols * r1; it += nt) {
     const int cl = it % kSpCols, k1 = it / kSpCols;
     if (cl < ncol) {
+      const int vc = slab_column(p, c0 + cl);
       with_radix<0>(r2, [&](auto rc_) {
         constexpr int RR = decltype(rc_)::value;
         C2<T> u[RR], d[RR];
@@ -95,7 +95,7 @@ k_z_spinor(LocalPlan p, int nbc, const T* __restrict__ vu, const T* __restrict__
         DFT<RR, +1, T>::run(d);
 #pragma unroll
         for (int a = 0; a < RR; ++a) {
-          const size_t o = (size_t)(k1 + r1 * a) * p.plane + c0 + cl;
+          const size_t o = (size_t)(k1 + r1 * a) * p.plane + vc;
           const T a11 = vu[o], a22 = vd[o], xr = vr[o], xi = vi[o];
           const C2<T> pu = u[a], pd = d[a];
           // up' = (V1+V2) up + (V3 - i V4) down ; down' = (V1-V2) down + (V3 + i V4) up
@@ -199,10 +199,6 @@ int spin_local(cpw_b200_ctx* c, int nb, const C2<double>* psi, long long ldpsi, 
   const int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)nb, c->slab_budget / (2 * per_band)));
   if (int s = c->slab.ensure(2 * per_band * (size_t)chunk)) return s;
   W = (C2<T>*)c->slab.p;
-  const size_t sm_pl = smem_planes<T>(p);
-  auto* kc = kern::k_fwd_xy<T, 0, 0, 0, 0, 0>;
-  if ((e = smem_limit((const void*)kc, (size_t)sm_pl)) != cudaSuccess)
-    return cuda_fail(e, "hk_psi_spin attribute");
   const size_t sm_z = sizeof(C2<T>) * (2 * (size_t)p.n3 * kSpCols + p.n3);
   if ((e = smem_limit((const void*)k_z_spinor<T>, (size_t)sm_z)) != cudaSuccess)
     return cuda_fail(e, "hk_psi_spin attribute");
@@ -216,10 +212,11 @@ int spin_local(cpw_b200_ctx* c, int nb, const C2<double>* psi, long long ldpsi, 
     }
     k_z_spinor<T><<<dim3(tiles, nbc), kSpThreads, sm_z, st>>>(p, nbc, (const T*)v[0].p, (const T*)v[1].p,
                                                                (const T*)v[2].p, (const T*)v[3].p, tw[2], W);
-    for (int comp = 0; comp < 2; ++comp)
-      kc<<<dim3(p.nz, nbc), kern::kThreadsPlanes, sm_pl, st>>>(p, b0, psi + comp, ldpsi, hpsi + comp, ldh, ps, idx2,
-                                                               pos, ek2, tw[0], tw[1],
-                                                               W + (size_t)comp * nbc * p.nz * p.plane);
+    for (int comp = 0; comp < 2; ++comp) {
+      e = launch_forward_xy<T>(p, nbc, b0, psi + comp, ldpsi, hpsi + comp, ldh, ps, idx2, pos, ek2, tw[0], tw[1],
+                               W + (size_t)comp * nbc * p.nz * p.plane, st);
+      if (e != cudaSuccess) return cuda_fail(e, "hk_psi_spin forward xy");
+    }
     if ((e = cudaGetLastError()) != cudaSuccess) return cuda_fail(e, "hk_psi_spin kernels");
   }
   return kOk;
