@@ -205,6 +205,11 @@ struct cpw_b200_ctx {
   int nanl_sp = 0;
   cpwb::DevBuf anl_sp, anld_sp, sp_idx2, sp_ek2;
 
+  // adjoint calls: work space and the complex transform of the box, kept between calls
+  cpwb::DevBuf adj;
+  void* fft_plan = nullptr;
+  int fft_n[3] = {0, 0, 0};
+
   // poll limit of the eigensolver's cooperative grid barrier (bounded device wait)
   long long grid_polls = 1LL << 24;
   // eigensolver device buffers and cuSOLVER handle, kept between calls (ditsp.cu)
@@ -236,6 +241,7 @@ inline void projectors_changed(cpw_b200_ctx* c) {
   c->crt_off = false;
 }
 void ditsp_release(cpw_b200_ctx* c);
+void adjoint_release(cpw_b200_ctx* c);
 int ctx_set_potential_spin(cpw_b200_ctx* c, const double* vscr_sp, long long mxdscr, int nsp);
 int ctx_set_projectors_spin(cpw_b200_ctx* c, int nanl, const double* anlsp, long long ld, const double* xnlkb);
 int ctx_hkpsi_kin_device(cpw_b200_ctx* c, int nb, const void* psi, long long ldpsi, void* hpsi, long long ldh,
