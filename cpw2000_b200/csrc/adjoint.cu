@@ -32,7 +32,17 @@ using Z = cuDoubleComplex;
 constexpr int kDensThreads = 256;
 constexpr int kDensCB = 32;
 
-// inverse z of the kept planes of every band of the chunk, |.|^2 accumulated with
+// rho += the band groups' boxes, in order
+__global__ void k_add_boxes(long long n, int groups, const double* __restrict__ part, double* __restrict__ rho) {
+  for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
+    double s = rho[t];
+    for (int g = 0; g < groups; ++g) s += part[(size_t)g * n + t];
+    rho[t] = s;
+  }
+}
+
+// Run-time form of the density's z stage (line lengths without a compiled one, hkpsi_kernels.cuh): inverse z
+// of the kept planes of every band of the chunk, |.|^2 accumulated with
 // the band weights; one CTA per 32 xy-columns; rho += the chunk's contribution
 __global__ void __launch_bounds__(kDensThreads)
 k_dens_z(LocalPlan p, int nbc, const double* __restrict__ occ, const C2<double>* __restrict__ twz,
@@ -324,8 +334,13 @@ int density_device(cpw_b200_ctx* c, int nb, const void* psi, long long ldpsi, co
   const int chunk = (int)std::max<size_t>(1, std::min<size_t>((size_t)nb, c->slab_budget / per_band));
   int s;
   if ((s = c->slab.ensure(per_band * (size_t)chunk))) return s;
-  if ((s = c->adj.ensure(sizeof(double) * nb))) return s;
+  // small boxes have few column tiles: their bands are split over groups of CTAs, each with its own box
+  const long long box = p.plane * p.n3, tiles = (p.plane + 15) / 16;
+  const int groups = has_line_form(p) ? (int)std::max(1LL, std::min<long long>(std::min(chunk, 8), 592 / tiles)) : 1;
+  const size_t occ_bytes = (sizeof(double) * (size_t)nb + 255) & ~(size_t)255;
+  if ((s = c->adj.ensure(occ_bytes + (groups > 1 ? sizeof(double) * (size_t)groups * box : 0)))) return s;
   const double* docc = (const double*)c->adj.p;
+  double* part = groups > 1 ? (double*)((char*)c->adj.p + occ_bytes) : nullptr;
   if ((e = cudaMemcpyAsync(c->adj.p, occ, sizeof(double) * nb, cudaMemcpyHostToDevice, st)) != cudaSuccess)
     return cuda_fail(e, "density occ");
   const size_t sm = (sizeof(C2<double>) + sizeof(double)) * (size_t)p.n3 * kDensCB + sizeof(C2<double>) * p.n3;
@@ -337,6 +352,16 @@ int density_device(cpw_b200_ctx* c, int nb, const void* psi, long long ldpsi, co
                                   (const int*)c->pw_idx.p, (const int*)c->pw_pos.p, (const C2<double>*)c->tw64[0].p,
                                   (const C2<double>*)c->tw64[1].p, (C2<double>*)c->slab.p, st);
     if (e != cudaSuccess) return cuda_fail(e, "density inverse xy");
+    if (has_line_form(p)) {
+      e = launch_density_z(p, nbc, groups, docc + b0, (const C2<double>*)c->tw64[2].p, (const C2<double>*)c->slab.p,
+                           (double*)rho, part, st);
+      if (e == cudaSuccess && groups > 1) {
+        k_add_boxes<<<1184, 256, 0, st>>>(box, groups, part, (double*)rho);
+        e = cudaGetLastError();
+      }
+      if (e != cudaSuccess) return cuda_fail(e, "density z");
+      continue;
+    }
     const unsigned grid = (unsigned)((p.plane + kDensCB - 1) / kDensCB);
     k_dens_z<<<grid, kDensThreads, sm, st>>>(p, nbc, docc + b0, (const C2<double>*)c->tw64[2].p,
                                              (const C2<double>*)c->slab.p, (double*)rho);

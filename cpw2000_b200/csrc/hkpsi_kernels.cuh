@@ -415,11 +415,10 @@ k_z_vloc_pipe(LocalPlan p, int nbc, int bands_per_group, const T* __restrict__ v
 // last pass, and needs two barriers per band: what pass 1 of band b + 1 overwrites in shared memory the
 // same thread has read in the last pass of band b.
 // ---------------------------------------------------------------------------
-template <typename T, int R1, int R2, int CB> constexpr int z_min_blocks() {
-  return std::max(1, 65536 / (CB * R2 * (sizeof(T) == 8 ? 112 : 64)));
-}
+// CTAs per SM asked of the register allocator for a thread budget of `regs` registers
+template <int R2, int CB> constexpr int z_min_blocks(int regs) { return std::max(1, 65536 / (CB * R2 * regs)); }
 template <typename T, int R1, int R2, int CB>
-__global__ void __launch_bounds__(CB * R2, (z_min_blocks<T, R1, R2, CB>()))
+__global__ void __launch_bounds__(CB * R2, (z_min_blocks<R2, CB>(sizeof(T) == 8 ? 112 : 64)))
 k_z_band(LocalPlan p, int nbc, int per, const T* __restrict__ vr, const C2<T>* __restrict__ twz, C2<T>* __restrict__ W) {
   constexpr int N3 = R1 * R2, NT = CB * R2, Q = quarter(R1);
   extern __shared__ __align__(16) unsigned char smem_raw[];
@@ -504,6 +503,181 @@ k_z_band(LocalPlan p, int nbc, int per, const T* __restrict__ vr, const C2<T>* _
 }
 template <typename T, int R1, int R2, int CB> constexpr size_t smem_z_band() {
   return (size_t)R1 * R2 * (CB * (sizeof(C2<T>) + sizeof(T)) + sizeof(C2<T>));
+}
+
+// The inverse half of B for the density: rho(r) += sum_b occ_b |psi_b(r)|^2. Thread and memory layout of
+// k_z_band; the sum over the CTA's bands of a point stays in a register of the thread that owns its
+// line in the second pass. part: null = add to rho, else the band groups' own boxes (summed by the caller).
+template <int R1, int R2, int CB>
+__global__ void __launch_bounds__(CB * R2, (z_min_blocks<R2, CB>(128)))
+k_z_density(LocalPlan p, int nbc, int per, const double* __restrict__ occ, const C2<double>* __restrict__ twz,
+            const C2<double>* __restrict__ W, double* __restrict__ rho, double* __restrict__ part) {
+  using T = double;
+  constexpr int N3 = R1 * R2, NT = CB * R2, Q = quarter(R1);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C2<T>* Cs = reinterpret_cast<C2<T>*>(smem_raw);
+  C2<T>* sz = Cs + N3 * CB;
+  const int tid = threadIdx.x, cl = tid % CB, j = tid / CB;
+  const size_t pl = (size_t)p.plane;
+  const long long col = (long long)blockIdx.x * CB + cl;
+  const bool ok = col < p.plane;
+  const int b_lo = blockIdx.y * per, b_hi = min(nbc, b_lo + per);
+  const int kd = p.kd3, skip = N3 - p.nz;
+  const size_t band = (size_t)p.nz * pl;
+  const C2<T>* Wb = W + (size_t)b_lo * band + col;
+  C2<T> nx[2 * Q];
+  auto load = [&](const C2<T>* w) {
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const int z = R2 * q + j, zh = R2 * (R1 - Q + q) + j;
+      nx[q] = ok && z <= kd ? w[z * pl] : czero<T>();
+      nx[Q + q] = ok && zh >= N3 - kd ? w[(zh - skip) * pl] : czero<T>();
+    }
+  };
+  if (b_lo < b_hi) load(Wb);
+  for (int i = tid; i < N3; i += NT) sz[i] = twz[i];
+  T acc[R2];
+#pragma unroll
+  for (int a = 0; a < R2; ++a) acc[a] = T(0);
+  __syncthreads();
+  for (int b = b_lo; b < b_hi; ++b, Wb += band) {
+    {
+      C2<T> v[R1];
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        v[q] = nx[q];
+        v[R1 - Q + q] = nx[Q + q];
+      }
+      DFTM<quarter_bits(R1), R1, +1, T>::run(v);
+#pragma unroll
+      for (int a = 0; a < R1; ++a) Cs[(R2 * a + j) * CB + cl] = a == 0 ? v[0] : cmulc<T>(v[a], sz[j * a]);
+    }
+    if (b + 1 < b_hi) load(Wb + band);
+    const T f = occ[b];
+    __syncthreads();
+    if (R1 == R2 || j < R1) {
+      C2<T> v[R2];
+#pragma unroll
+      for (int a = 0; a < R2; ++a) v[a] = Cs[(R2 * j + a) * CB + cl];
+      DFT<R2, +1, T>::run(v);
+#pragma unroll
+      for (int a = 0; a < R2; ++a) acc[a] += f * (v[a].x * v[a].x + v[a].y * v[a].y);
+    }
+    __syncthreads();
+  }
+  if (ok && (R1 == R2 || j < R1)) {
+    const int vc = slab_column(p, col);
+#pragma unroll
+    for (int a = 0; a < R2; ++a) {
+      const size_t o = (j + R1 * a) * pl + vc;
+      if (part)
+        part[(size_t)blockIdx.y * N3 * pl + o] = acc[a];
+      else
+        rho[o] += acc[a];
+    }
+  }
+}
+
+// The non-collinear z stage of one spinor per step: both components' columns are transformed, multiplied by
+// [[V1+V2, V3-iV4], [V3+iV4, V1-V2]] and transformed back. One thread per (component, line, column); the
+// four potential columns are staged once per CTA and serve its bands, the kept points of the next spinor
+// are loaded while this one is transformed. Up slabs at W, down slabs nbc slabs later.
+template <typename T, int R1, int R2, int CB>
+__global__ void __launch_bounds__(2 * CB * R2, (z_min_blocks<R2, 2 * CB>(sizeof(T) == 8 ? 168 : 96)))
+k_z_spinor_band(LocalPlan p, int nbc, int per, const T* __restrict__ vu, const T* __restrict__ vd,
+                const T* __restrict__ vr, const T* __restrict__ vi, const C2<T>* __restrict__ twz, C2<T>* __restrict__ W) {
+  constexpr int N3 = R1 * R2, NT = 2 * CB * R2, Q = quarter(R1);
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  C2<T>* Call = reinterpret_cast<C2<T>*>(smem_raw);          // [component][z][column]
+  C2<T>* sz = Call + 2 * N3 * CB;
+  T* Vs = reinterpret_cast<T*>(sz + N3);                     // [vu, vd, vr, vi][z][column]
+  const int tid = threadIdx.x, cl = tid % CB, j = (tid / CB) % R2, s = tid / (CB * R2);
+  const size_t pl = (size_t)p.plane;
+  const long long col = (long long)blockIdx.x * CB + cl;
+  const bool ok = col < p.plane;
+  const int b_lo = blockIdx.y * per, b_hi = min(nbc, b_lo + per);
+  if (b_lo >= b_hi) return;
+  const int kd = p.kd3, skip = N3 - p.nz;
+  const size_t band = (size_t)p.nz * pl;
+  C2<T>* Cs = Call + s * N3 * CB;
+  const C2<T>* Co = Call + (1 - s) * N3 * CB;
+  C2<T>* Wb = W + ((size_t)s * nbc + b_lo) * band + col;
+  C2<T> nx[2 * Q];
+  auto load = [&](const C2<T>* w) {
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const int z = R2 * q + j, zh = R2 * (R1 - Q + q) + j;
+      nx[q] = ok && z <= kd ? w[z * pl] : czero<T>();
+      nx[Q + q] = ok && zh >= N3 - kd ? w[(zh - skip) * pl] : czero<T>();
+    }
+  };
+  load(Wb);
+  for (int i = tid; i < N3; i += NT) sz[i] = twz[i];
+  {
+    const int vc = ok ? slab_column(p, col) : 0;
+    const T* src[4] = {vu, vd, vr, vi};
+#pragma unroll
+    for (int k = 0; k < 2; ++k)
+      for (int z = j; z < N3; z += R2) Vs[((2 * s + k) * N3 + z) * CB + cl] = ok ? src[2 * s + k][z * pl + vc] : T(0);
+  }
+  __syncthreads();
+  const T* Va = Vs + s * N3 * CB;                            // this component's diagonal term
+  const T* Vr = Vs + 2 * N3 * CB;
+  const T* Vi = Vr + N3 * CB;
+  const T sgn = s == 0 ? T(1) : T(-1);                       // V3 - i V4 acts on down, V3 + i V4 on up
+  for (int b = b_lo; b < b_hi; ++b, Wb += band) {
+    {
+      C2<T> v[R1];
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        v[q] = nx[q];
+        v[R1 - Q + q] = nx[Q + q];
+      }
+      DFTM<quarter_bits(R1), R1, +1, T>::run(v);
+#pragma unroll
+      for (int a = 0; a < R1; ++a) Cs[(R2 * a + j) * CB + cl] = a == 0 ? v[0] : cmulc<T>(v[a], sz[j * a]);
+    }
+    if (b + 1 < b_hi) load(Wb + band);
+    __syncthreads();
+    C2<T> v[R2];
+    const bool mid = R1 == R2 || j < R1;
+    if (mid) {
+#pragma unroll
+      for (int a = 0; a < R2; ++a) v[a] = Cs[(R2 * j + a) * CB + cl];
+      DFT<R2, +1, T>::run(v);
+#pragma unroll
+      for (int a = 0; a < R2; ++a) Cs[(R2 * j + a) * CB + cl] = v[a];
+    }
+    __syncthreads();
+    if (mid) {
+#pragma unroll
+      for (int a = 0; a < R2; ++a) {
+        const C2<T> o = Co[(R2 * j + a) * CB + cl];
+        const int z = (j + R1 * a) * CB + cl;
+        const T d = Va[z], xr = Vr[z], xi = sgn * Vi[z];
+        v[a] = mk<T>(d * v[a].x + xr * o.x - xi * o.y, d * v[a].y + xr * o.y + xi * o.x);
+      }
+      DFT<R2, -1, T>::run(v);
+    }
+    __syncthreads();
+    if (mid) {
+#pragma unroll
+      for (int a = 0; a < R2; ++a) Cs[(R2 * j + a) * CB + cl] = a == 0 ? v[0] : cmul<T>(v[a], sz[j * a]);
+    }
+    __syncthreads();
+    {
+      C2<T> w[R1];
+#pragma unroll
+      for (int a = 0; a < R1; ++a) w[a] = Cs[(R2 * a + j) * CB + cl];
+      DFT<R1, -1, T>::run(w);
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const int z = R2 * q + j, zh = R2 * (R1 - Q + q) + j;
+        if (ok && z <= kd) Wb[z * pl] = w[q];
+        if (ok && zh >= N3 - kd) Wb[(zh - skip) * pl] = w[R1 - Q + q];
+      }
+    }
+  }
 }
 
 // ---------------------------------------------------------------------------
@@ -776,6 +950,36 @@ cudaError_t launch_z_impl(const LocalPlan& p, int nbc, const T* vr, const C2<T>*
   return cudaGetLastError();
 }
 
+// Launch the density's z stage. groups: band groups (part holds a box for each when there are several).
+template <int R1, int R2>
+cudaError_t launch_density_impl(const LocalPlan& p, int nbc, int groups, const double* occ, const C2<double>* twz,
+                                const C2<double>* W, double* rho, double* part, cudaStream_t st) {
+  constexpr int CB = 16;
+  constexpr size_t sm = (size_t)R1 * R2 * (CB + 1) * sizeof(C2<double>);
+  auto* k = k_z_density<R1, R2, CB>;
+  cudaError_t e = smem_limit((const void*)k, sm);
+  if (e != cudaSuccess) return e;
+  const int per = (nbc + groups - 1) / groups;
+  k<<<dim3((unsigned)((p.plane + CB - 1) / CB), groups), CB * R2, sm, st>>>(p, nbc, per, occ, twz, W, rho, part);
+  return cudaGetLastError();
+}
+
+// Launch the non-collinear z stage for a z split R1 x R2.
+template <typename T, int R1, int R2>
+cudaError_t launch_spinor_impl(const LocalPlan& p, int nbc, const T* vu, const T* vd, const T* vr, const T* vi,
+                               const C2<T>* twz, C2<T>* W, int nsm, cudaStream_t st) {
+  constexpr int CB = 8;
+  constexpr size_t sm = (size_t)R1 * R2 * (CB * (2 * sizeof(C2<T>) + 4 * sizeof(T)) + sizeof(C2<T>));
+  auto* k = k_z_spinor_band<T, R1, R2, CB>;
+  cudaError_t e = smem_limit((const void*)k, sm);
+  if (e != cudaSuccess) return e;
+  const long long tiles = (p.plane + CB - 1) / CB;
+  const int g = band_groups(p, tiles, nbc, nsm), per = (nbc + g - 1) / g;
+  k<<<dim3((unsigned)tiles, (unsigned)((nbc + per - 1) / per)), 2 * CB * R2, sm, st>>>(p, nbc, per, vu, vd, vr, vi, twz,
+                                                                                  W);
+  return cudaGetLastError();
+}
+
 }  // namespace kern
 
 #define CPWB_INV_ARGS(T)                                                                                     \
@@ -798,6 +1002,13 @@ cudaError_t launch_z_impl(const LocalPlan& p, int nbc, const T* vr, const C2<T>*
 #define CPWB_PLANES(EXTERN, T, R1, R2, TC)                                                           \
   EXTERN template cudaError_t kern::launch_a_impl<T, R1, R2, R1, R2, TC>(CPWB_INV_ARGS(T));          \
   EXTERN template cudaError_t kern::launch_c_impl<T, R1, R2, R1, R2, TC>(CPWB_C_ARGS(T));
-#define CPWB_LINES(EXTERN, T, R1, R2) EXTERN template cudaError_t kern::launch_z_impl<T, R1, R2>(CPWB_Z_ARGS(T));
+#define CPWB_LINES(EXTERN, T, R1, R2)                                                                       \
+  EXTERN template cudaError_t kern::launch_z_impl<T, R1, R2>(CPWB_Z_ARGS(T));                               \
+  EXTERN template cudaError_t kern::launch_spinor_impl<T, R1, R2>(                                          \
+      const LocalPlan&, int, const T*, const T*, const T*, const T*, const C2<T>*, C2<T>*, int, cudaStream_t);
+#define CPWB_DENSITY(EXTERN, R1, R2)                                                                        \
+  EXTERN template cudaError_t kern::launch_density_impl<R1, R2>(const LocalPlan&, int, int, const double*,  \
+                                                                const C2<double>*, const C2<double>*,       \
+                                                                double*, double*, cudaStream_t);
 
 }  // namespace cpwb

@@ -16,7 +16,8 @@ CPWB_FOR_PLANES(CPWB_DECLARE)
 #undef CPWB_DECLARE
 CPWB_PLANES(extern, double, 0, 0, 0)
 CPWB_PLANES(extern, float, 0, 0, 0)
-#define CPWB_DECLARE(R1, R2) CPWB_LINES(extern, double, R1, R2) CPWB_LINES(extern, float, R1, R2)
+#define CPWB_DECLARE(R1, R2) \
+  CPWB_LINES(extern, double, R1, R2) CPWB_LINES(extern, float, R1, R2) CPWB_DENSITY(extern, R1, R2)
 CPWB_FOR_LINES(CPWB_DECLARE)
 #undef CPWB_DECLARE
 
@@ -84,6 +85,42 @@ static cudaError_t launch_z(const LocalPlan& p, int nbc, const T* vr, const C2<T
   }
   return cudaGetLastError();
 }
+
+bool has_line_form(const LocalPlan& p) {
+  if (!in_quarters(p.kd3, p.dz.r1, p.dz.r2)) return false;
+#define CPWB_TRY(R1, R2) \
+  if (is_split(p.dz, R1, R2)) return true;
+  CPWB_FOR_LINES(CPWB_TRY)
+#undef CPWB_TRY
+  return false;
+}
+
+cudaError_t launch_density_z(const LocalPlan& p, int nbc, int groups, const double* occ, const C2<double>* twz,
+                             const C2<double>* W, double* rho, double* part, cudaStream_t st) {
+#define CPWB_TRY(R1, R2) \
+  if (is_split(p.dz, R1, R2)) return kern::launch_density_impl<R1, R2>(p, nbc, groups, occ, twz, W, rho, part, st);
+  CPWB_FOR_LINES(CPWB_TRY)
+#undef CPWB_TRY
+  return cudaErrorInvalidValue;
+}
+
+template <typename T>
+cudaError_t launch_spinor_z(const LocalPlan& p, int nbc, const T* vu, const T* vd, const T* vr, const T* vi,
+                            const C2<T>* twz, C2<T>* W, cudaStream_t st) {
+  int nsm = 148, dev = 0;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev);
+#define CPWB_TRY(R1, R2) \
+  if (is_split(p.dz, R1, R2)) return kern::launch_spinor_impl<T, R1, R2>(p, nbc, vu, vd, vr, vi, twz, W, nsm, st);
+  CPWB_FOR_LINES(CPWB_TRY)
+#undef CPWB_TRY
+  return cudaErrorInvalidValue;
+}
+#define CPWB_SPINOR(T)                                                                                      \
+  template cudaError_t launch_spinor_z<T>(const LocalPlan&, int, const T*, const T*, const T*, const T*,    \
+                                          const C2<T>*, C2<T>*, cudaStream_t);
+CPWB_SPINOR(double)
+CPWB_SPINOR(float)
 
 template <typename T>
 cudaError_t launch_local(const LocalPlan& p, int nbc, int band0, const C2<double>* psi, long long ldpsi,

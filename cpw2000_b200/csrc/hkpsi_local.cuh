@@ -162,4 +162,15 @@ cudaError_t launch_forward_xy(const LocalPlan& p, int nbc, int band0, const C2<d
                               const int* pw_pos, const double* ekpg, const C2<T>* twx, const C2<T>* twy,
                               const C2<T>* W, cudaStream_t st);
 
+// The register forms of the z stages exist for the plan's z lines (compiled length, kept planes in the
+// outer quarters of the line). Only then may the next two be called:
+bool has_line_form(const LocalPlan& p);
+// the density's (groups band groups; part: a box each when there are several, else null and rho is added to)
+cudaError_t launch_density_z(const LocalPlan& p, int nbc, int groups, const double* occ, const C2<double>* twz,
+                             const C2<double>* W, double* rho, double* part, cudaStream_t st);
+// the non-collinear one (down slabs nbc slabs after the up slabs)
+template <typename T>
+cudaError_t launch_spinor_z(const LocalPlan& p, int nbc, const T* vu, const T* vd, const T* vr, const T* vi,
+                            const C2<T>* twz, C2<T>* W, cudaStream_t st);
+
 }  // namespace cpwb

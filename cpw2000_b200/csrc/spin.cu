@@ -34,8 +34,8 @@ __global__ void k_double_index(int m, const int* __restrict__ idx, const double*
   }
 }
 
-// z stage of the nsp = 4 form for one tile of kSpCols xy columns of one spinor: up slab of
-// spinor b at W[b], down slab at W[nbc + b]. Potentials pre-scaled by 1/N in [z][y][x] order:
+// Run-time form of the nsp = 4 z stage (line lengths without a compiled one, hkpsi_kernels.cuh) for one
+// tile of kSpCols xy columns of one spinor: up slab of spinor b at W[b], down slab at W[nbc + b]. Potentials pre-scaled by 1/N in [z][y][x] order:
 // vu = V1+V2, vd = V1-V2, and the off-diagonal V3 - iV4 = vr + i vi.
 template <typename T>
 __global__ void __launch_bounds__(kSpThreads)
@@ -210,8 +210,13 @@ int spin_local(cpw_b200_ctx* c, int nb, const C2<double>* psi, long long ldpsi, 
                                W + (size_t)comp * nbc * p.nz * p.plane, st);
       if (e != cudaSuccess) return cuda_fail(e, "hk_psi_spin inverse xy");
     }
-    k_z_spinor<T><<<dim3(tiles, nbc), kSpThreads, sm_z, st>>>(p, nbc, (const T*)v[0].p, (const T*)v[1].p,
-                                                               (const T*)v[2].p, (const T*)v[3].p, tw[2], W);
+    if (has_line_form(p)) {
+      e = launch_spinor_z<T>(p, nbc, (const T*)v[0].p, (const T*)v[1].p, (const T*)v[2].p, (const T*)v[3].p, tw[2], W, st);
+      if (e != cudaSuccess) return cuda_fail(e, "hk_psi_spin z stage");
+    } else {
+      k_z_spinor<T><<<dim3(tiles, nbc), kSpThreads, sm_z, st>>>(p, nbc, (const T*)v[0].p, (const T*)v[1].p,
+                                                                 (const T*)v[2].p, (const T*)v[3].p, tw[2], W);
+    }
     for (int comp = 0; comp < 2; ++comp) {
       e = launch_forward_xy<T>(p, nbc, b0, psi + comp, ldpsi, hpsi + comp, ldh, ps, idx2, pos, ek2, tw[0], tw[1],
                                W + (size_t)comp * nbc * p.nz * p.plane, st);
