@@ -213,7 +213,7 @@ struct cpw_b200_ctx {
   // poll limit of the eigensolver's cooperative grid barrier (bounded device wait)
   long long grid_polls = 1LL << 24;
   // eigensolver device buffers and cuSOLVER handle, kept between calls (ditsp.cu)
-  cpwb::DevBuf ditsp_pool[24];
+  cpwb::DevBuf ditsp_pool[22];
   void* ditsp_sol = nullptr;
 
   cpwb::StageTimer timer;

@@ -8,6 +8,7 @@
 // context's operator (FP64 drop-in or the mixed-precision form).
 #include <cusolverDn.h>
 #include <math.h>
+#include <stddef.h>
 #include <stdio.h>
 #include <stdlib.h>
 #include <string.h>
@@ -263,6 +264,197 @@ __global__ void __launch_bounds__(256) k_mgs(MgsArgs a) {
       if (hxi) hxi[r] = make_cuDoubleComplex(hxi[r].x * suma, hxi[r].y * suma);
     }
   }
+}
+
+// The same steps with the same partial sums, added in the same order (bit for bit the grid form's result),
+// by one cluster. A block of 256 threads plays one CTA of the grid form (up to 512 rows, two a thread, the
+// current vector in registers), V blocks to a CTA. The blocks' sums cross the CTAs by stores to distributed
+// shared memory and an mbarrier of each CTA that counts the blocks' arrivals. Bound: the chain of
+// nvec (nvec + 1) / 2 sums, each two shuffle trees and one trip between SMs. An mbarrier wait is limited
+// like the grid barrier's (polls); every CTA, also one that gave up, ends in the cluster barrier, so none
+// leaves while another may still store to its shared memory.
+constexpr int kMgsRows = 512, kMgsCtas = 8, kMgsBlocks = 4;
+
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.aligned;\nbarrier.cluster.wait.aligned;\n" ::: "memory");
+}
+__device__ __forceinline__ unsigned peer_address(const void* p, unsigned rank) {
+  unsigned r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(r) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ bool phase_done(const unsigned long long* bar, unsigned parity) {
+  unsigned ok;
+  asm volatile(
+      "{\n.reg .pred p;\nmbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\nselp.u32 %0, 1, 0, p;\n}\n"
+      : "=r"(ok)
+      : "r"((unsigned)__cvta_generic_to_shared(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
+
+template <int V> __global__ void __launch_bounds__(256 * V) k_mgs_cluster(MgsArgs a, int blocks) {
+  __shared__ double sh[V][3][8];
+  __shared__ double slot[2][kMgsCtas * V][3];
+  __shared__ __align__(8) unsigned long long bar[2];
+  const int lane = threadIdx.x & 31, tid = threadIdx.x & 255, vb = threadIdx.x >> 8, w = tid >> 5;
+  const int blk = blockIdx.x * V + vb;
+  const int per = (a.m + blocks - 1) / blocks, r0 = blk * per, rows = blk < blocks ? max(0, min(a.m, r0 + per) - r0) : 0;
+  const bool has[2] = {tid < rows, tid + 256 < rows};
+  if (threadIdx.x == 0) {
+    for (int p = 0; p < 2; ++p)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"((unsigned)__cvta_generic_to_shared(&bar[p])),
+                   "r"(blocks)
+                   : "memory");
+    asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
+  }
+  cluster_sync();
+
+  int round = 0;
+  // the block's sums of k values, to every CTA of the cluster
+  auto post = [&](const double* v, int k) {
+    const int par = round & 1;
+    for (int t = 0; t < k; ++t) {
+      double s = v[t];
+      for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+      if (lane == 0) sh[vb][t][w] = s;
+    }
+    if (V == 1) __syncthreads();
+    else asm volatile("bar.sync %0, 256;\n" ::"r"(vb + 1) : "memory");   // the block's own barrier
+    if (w == 0 && blk < blocks) {
+      double tot[3];
+      for (int t = 0; t < k; ++t) {
+        double s = lane < 8 ? sh[vb][t][lane] : 0.0;
+        for (int o = 4; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+        tot[t] = __shfl_sync(0xffffffffu, s, 0);
+      }
+      if (lane < gridDim.x) {
+        const unsigned dst = peer_address(&slot[par][blk][0], lane);
+        for (int t = 0; t < k; ++t)
+          asm volatile("st.shared::cluster.f64 [%0], %1;\n" ::"r"(dst + 8 * t), "d"(tot[t]) : "memory");
+        asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(peer_address(&bar[par], lane))
+                     : "memory");
+      }
+    }
+  };
+  // waits for the blocks' sums and adds them; false (for the whole CTA) when they did not come in time
+  auto collect = [&](double* o, int k) {
+    const int par = round & 1;
+    bool ok = true;
+    if (threadIdx.x == 32)   // one poller, in a warp that does not post
+      for (long long it = 0; !phase_done(&bar[par], (round >> 1) & 1);)
+        if (++it > a.spin_limit) {
+          ok = false;
+          break;
+        }
+    if (!__syncthreads_and(ok)) {
+      if (threadIdx.x == 0) atomicExch(a.err, 1);
+      return false;
+    }
+    for (int t = 0; t < k; ++t) {
+      double s = lane < blocks ? slot[par][lane][t] : 0.0;
+      for (int q = 16; q > 0; q >>= 1) s += __shfl_down_sync(0xffffffffu, s, q);
+      o[t] = __shfl_sync(0xffffffffu, s, 0);
+    }
+    ++round;
+    return true;
+  };
+  auto load = [&](const Z* x, int i, Z* q) {
+    const Z* p = x + (size_t)i * a.m + r0 + tid;
+    for (int r = 0; r < 2; ++r) q[r] = has[r] ? p[256 * r] : make_cuDoubleComplex(0.0, 0.0);
+  };
+  auto dot = [&](const Z* p, const Z* q, double& re, double& im) {
+    re = 0;
+    im = 0;
+#pragma unroll
+    for (int r = 0; r < 2; ++r)
+      if (has[r]) {
+        const Z u = p[r], w = q[r];
+        re += u.x * w.x + u.y * w.y;
+        im += u.x * w.y - u.y * w.x;
+      }
+  };
+  auto axpy = [&](const Z* p, Z* q, double cr, double ci) {   // q -= c p
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const Z u = p[r];
+      q[r] = make_cuDoubleComplex(q[r].x - (cr * u.x - ci * u.y), q[r].y - (cr * u.y + ci * u.x));
+    }
+  };
+  auto steps = [&]() {
+    double v[3], o[3];
+    for (int i = 0; i < a.nvec; ++i) {
+      Z xi[2], hi[2], xj[2], nx[2], hj[2];
+      load(a.x, i, xi);
+      if (a.also) load(a.hx, i, hi);
+      if (i > 0) {
+        double xni = 0, xnp = 0;
+        load(a.x, 0, xj);
+        for (int pass = 0; pass < 2; ++pass) {
+          for (int j = 0; j < i; ++j) {
+            const bool first = pass == 0 && j == 0;
+            dot(xj, xi, v[0], v[1]);
+            if (first) {   // xni on the vector before any projection
+              double im;
+              dot(xi, xi, v[2], im);
+            }
+            post(v, first ? 3 : 2);
+            load(a.x, j + 1 < i ? j + 1 : 0, nx);
+            if (a.also) load(a.hx, j, hj);
+            if (!collect(o, first ? 3 : 2)) return;
+            if (first) xni = o[2];
+            if (pass == 0) xnp += o[0] * o[0] + o[1] * o[1];
+            axpy(xj, xi, o[0], o[1]);
+            if (a.also) axpy(hj, hi, o[0], o[1]);
+            for (int r = 0; r < 2; ++r) xj[r] = nx[r];
+          }
+          if (!(xnp > a.rep * xni)) break;
+        }
+      }
+      double im;
+      dot(xi, xi, v[0], im);
+      post(v, 1);
+      if (!collect(o, 1)) return;
+      double suma = o[0];
+      const double xs = a.xscl[i];
+      int keep = 1;
+      if (xs > a.peq) {
+        if (suma < a.eps * xs) {
+          suma = 0.0;
+          keep = 0;
+        } else {
+          suma = 1.0 / sqrt(suma);
+        }
+      } else {
+        suma = 0.0;
+        keep = 0;
+      }
+      if (blockIdx.x == 0 && threadIdx.x == 0 && !keep) a.irow[i] = 0;
+      for (int r = 0; r < 2; ++r)
+        if (has[r]) {
+          const size_t at = (size_t)i * a.m + r0 + tid + 256 * r;
+          a.x[at] = make_cuDoubleComplex(xi[r].x * suma, xi[r].y * suma);
+          if (a.also) a.hx[at] = make_cuDoubleComplex(hi[r].x * suma, hi[r].y * suma);
+        }
+    }
+  };
+  steps();
+  __syncwarp();
+  cluster_sync();
+}
+
+template <int V> cudaError_t launch_mgs_cluster(const MgsArgs& a, int blocks, cudaStream_t st) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((blocks + V - 1) / V);
+  cfg.blockDim = dim3(256 * V);
+  cfg.stream = st;
+  cudaLaunchAttribute at{};
+  at.id = cudaLaunchAttributeClusterDimension;
+  at.val.clusterDim.x = cfg.gridDim.x;
+  at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, k_mgs_cluster<V>, a, blocks);
 }
 
 // G (k x k, lower triangle used) of a block whose columns idx[0..nd) were zeroed: their rows and
@@ -717,7 +909,7 @@ struct Solver {
 
   // ---- block Gram-Schmidt family (grsch_mod / grsch_mm / grsch_loop / grsch_shift) ----
   // grsch_mod on the device (k_mgs); irow/xscl are host arrays of nvec entries
-  DevBuf mgs_part, mgs_bar, mgs_irow, mgs_xscl;
+  DevBuf mgs_part, mgs_io;
   int mgs_grid = 0;
   int grsch_mod(bool also, Z* x, Z* hx, int nvec, int* irow, const double* xscl) {
     if (nvec <= 0) return kOk;
@@ -732,36 +924,50 @@ struct Solver {
     }
     const int grid = std::max(1, std::min(mgs_grid, (m + 511) / 512));
     int s;
-    if ((s = mgs_part.ensure(sizeof(double) * 8 * (size_t)mgs_grid)) || (s = mgs_bar.ensure(sizeof(unsigned) * 4)) ||
-        (s = mgs_irow.ensure(sizeof(int) * 16)) || (s = mgs_xscl.ensure(sizeof(double) * 16)))
-      return s;
-    if ((s = ck(cudaMemsetAsync(mgs_bar.p, 0, sizeof(unsigned) * 4, st), "mgs"))) return s;
-    if ((s = ck(cudaMemcpyAsync(mgs_irow.p, irow, sizeof(int) * nvec, cudaMemcpyHostToDevice, st), "mgs"))) return s;
-    if ((s = ck(cudaMemcpyAsync(mgs_xscl.p, xscl, sizeof(double) * nvec, cudaMemcpyHostToDevice, st), "mgs")))
-      return s;
+    struct {             // one copy in, one out (of all but xscl)
+      unsigned bar[2];
+      int err, pad;
+      int irow[16];
+      double xscl[16];
+    } io{};
+    std::copy(irow, irow + nvec, io.irow);
+    std::copy(xscl, xscl + nvec, io.xscl);
+    if ((s = mgs_part.ensure(sizeof(double) * 8 * (size_t)mgs_grid)) || (s = mgs_io.ensure(sizeof io))) return s;
+    if ((s = ck(cudaMemcpyAsync(mgs_io.p, &io, sizeof io, cudaMemcpyHostToDevice, st), "mgs"))) return s;
+    char* dio = (char*)mgs_io.p;
     MgsArgs a;
     a.m = m;
     a.nvec = nvec;
     a.also = also ? 1 : 0;
     a.x = x;
     a.hx = hx;
-    a.xscl = (const double*)mgs_xscl.p;
-    a.irow = (int*)mgs_irow.p;
+    a.xscl = (const double*)(dio + offsetof(decltype(io), xscl));
+    a.irow = (int*)(dio + offsetof(decltype(io), irow));
     a.partial = (double*)mgs_part.p;
-    a.bar = (unsigned*)mgs_bar.p;
-    a.err = (int*)mgs_bar.p + 2;
+    a.bar = (unsigned*)dio;
+    a.err = (int*)(dio + offsetof(decltype(io), err));
     a.eps = CEPS20;
     a.peq = (1.0 / CEPS20) * 2.2250738585072014e-308;
     a.rep = C0P9999;
     a.spin_limit = c->grid_polls;
-    void* args[] = {&a};
-    if ((s = ck(cudaLaunchCooperativeKernel((const void*)k_mgs, dim3(grid), dim3(256), args, 0, st), "mgs launch")))
-      return s;
-    int err = 0;
-    if ((s = ck(cudaMemcpyAsync(irow, mgs_irow.p, sizeof(int) * nvec, cudaMemcpyDeviceToHost, st), "mgs"))) return s;
-    if ((s = ck(cudaMemcpyAsync(&err, (int*)mgs_bar.p + 2, sizeof(int), cudaMemcpyDeviceToHost, st), "mgs"))) return s;
+    // One cluster for 513 to 16,384 rows, what eight CTAs of four blocks hold (as few blocks to a CTA as that
+    // allows: 4,096 rows 37 us, two blocks 49 at 4,700, four 82 at 9,000; the grid form 91, 101 and 139); the
+    // grid form beyond, and for a block that one CTA holds, which waits for nobody. CPW_B200_MGS_GRID=1 keeps it.
+    const char* gv = getenv("CPW_B200_MGS_GRID");
+    if (!(gv && atoi(gv) != 0) && grid > 1 && grid == (m + kMgsRows - 1) / kMgsRows && grid <= kMgsCtas * kMgsBlocks) {
+      const cudaError_t e = grid <= kMgsCtas       ? launch_mgs_cluster<1>(a, grid, st)
+                            : grid <= 2 * kMgsCtas ? launch_mgs_cluster<2>(a, grid, st)
+                                                   : launch_mgs_cluster<4>(a, grid, st);
+      if ((s = ck(e, "mgs launch"))) return s;
+    } else {
+      void* args[] = {&a};
+      if ((s = ck(cudaLaunchCooperativeKernel((const void*)k_mgs, dim3(grid), dim3(256), args, 0, st), "mgs launch")))
+        return s;
+    }
+    if ((s = ck(cudaMemcpyAsync(&io, dio, offsetof(decltype(io), xscl), cudaMemcpyDeviceToHost, st), "mgs"))) return s;
     if ((s = ck(cudaStreamSynchronize(st), "mgs"))) return s;
-    if (err) return fail(kTimeout, "grsch_mod: a grid barrier wait gave up");
+    std::copy(io.irow, io.irow + nvec, irow);
+    if (io.err) return fail(kTimeout, "grsch_mod: a grid barrier wait gave up");
     return kOk;
   }
 
@@ -934,13 +1140,14 @@ struct Solver {
 // would serialise contexts that solve different k-points at the same time.
 struct SolverPool {
   Solver& S;
-  static constexpr int kN = 24;
+  static constexpr int kN = 22;
   DevBuf* m[kN];
   explicit SolverPool(Solver& s) : S(s) {
-    DevBuf* l[kN] = {&S.bas,  &S.hbas,      &S.smallA,    &S.smallV,   &S.dvec,     &S.dvec2,    &S.dz,
+    DevBuf* l[] = {&S.bas,  &S.hbas,      &S.smallA,    &S.smallV,   &S.dvec,     &S.dvec2,    &S.dz,
                      &S.work, &S.info,      &S.eg_d,      &S.hdiag_d,  &S.ham_prev, &S.chol_g,   &S.chol_work,
-                     &S.chol_info, &S.chol_idx, &S.mgs_part, &S.mgs_bar, &S.mgs_irow, &S.mgs_xscl, &S.chol_diag,
+                     &S.chol_info, &S.chol_idx, &S.mgs_part, &S.mgs_io, &S.chol_diag,
                      &S.chol_tmp, &S.chol_tri, &S.chol_lh};
+    static_assert(sizeof l == sizeof m && sizeof S.c->ditsp_pool == kN * sizeof(DevBuf), "one slot per buffer");
     for (int i = 0; i < kN; ++i) {
       m[i] = l[i];
       swap(*m[i], S.c->ditsp_pool[i]);
