@@ -15,16 +15,27 @@ namespace kern {
 
 constexpr int kThreadsPlanes = 256;
 constexpr int kThreadsCols = 256;
-// CTAs per SM asked of the register allocator: two CTAs of 320 threads or more (FP64 planes below), as many
-// as two of 384 in 80 registers.
-constexpr int pass_min_blocks(int nt) { return nt >= 320 ? 2 : 1; }
-// Kernels A and C: FP64 planes of 128 points or more take over 200 KB of shared memory (one CTA
-// per SM whatever the registers), so they get no register cap. The run-time form (n1 = 0) would take
-// the registers of its largest radix, one CTA of 256 threads per SM in FP64: it is held to two (FP32:
-// three), at the price of a few spills in radix 16.
-template <typename T> constexpr int plane_min_blocks(int nt, int n1) {
-  return n1 == 0 ? (sizeof(T) == 8 ? 2 : 3) : sizeof(T) == 8 && n1 >= 128 ? 1 : pass_min_blocks(nt);
+// CTAs per SM asked of the register allocator for kernels A and C (fwd): the passes wait on shared memory
+// and on the plane's loads, so small planes want as many CTAs as their shared memory lets in. us per launch
+// with this bound, before -> after:
+//   40 x 40 (320 threads; 2,560 bands FP32, 160 FP64): C FP32 three -> five 541 -> 404 (six the same), A FP32
+//   four -> six 361 -> 326; C FP64 two -> three 60 -> 52 (four 52 with the read-ahead gather that takes three
+//   to 46), A FP64 three -> four 36 -> 35.
+//   96 x 96 FP32 (160 bands): C with 384 threads in three CTAs 164, 256 in three 179, 256 in four 210;
+//   A in three 139, in four 160 (spills).
+//   FP64 planes of 128 points or more take over 200 KB of shared memory, one CTA per SM whatever the
+//   registers: no cap. The others: two CTAs of 384 threads in 80 registers.
+// The run-time form (n1 = 0) would take the registers of its largest radix, one CTA of 256 threads per SM in
+// FP64: it is held to two (three: 72 x 80 C 89 -> 105), in FP32 to three, or to five where a plane's shared
+// memory lets them in (many: 64 x 50, 91 bands, C 96 -> 83, A 81 -> 72; 48 bands of 48 x 48 42 -> 38 for
+// both, 72 x 72 76 -> 73; 80 x 80, which would hold four, 98 -> 111).
+template <typename T> constexpr int plane_min_blocks(int nt, int n1, bool fwd, bool many) {
+  if (n1 == 40) return sizeof(T) == 8 ? (fwd ? 3 : 4) : fwd ? 5 : 6;
+  if (n1 == 96 && sizeof(T) == 4) return 3;
+  if (n1 == 0) return sizeof(T) == 8 ? 2 : many ? 5 : 3;
+  return sizeof(T) == 8 && n1 >= 128 ? 1 : nt >= 320 ? 2 : 1;
 }
+constexpr size_t kManyPlaneBytes = 44 * 1024;   // five CTAs to an SM
 
 template <typename T> __device__ __forceinline__ C2<T> czero() { return mk<T>(T(0), T(0)); }
 
@@ -33,8 +44,8 @@ template <typename T> __device__ __forceinline__ C2<T> czero() { return mk<T>(T(
 // ---------------------------------------------------------------------------
 // PR: the kept x and y indices lie in the outer quarters of their lines (in_quarters below), so that
 // the first pass of each transform reads and multiplies those points alone.
-template <typename T, int RX1, int RX2, int RY1, int RY2, int TC, bool PR, int NT = kThreadsPlanes>
-__global__ void __launch_bounds__(NT, plane_min_blocks<T>(NT, RX1 * RX2))
+template <typename T, int RX1, int RX2, int RY1, int RY2, int TC, bool PR, int NT = kThreadsPlanes, bool MANY = false>
+__global__ void __launch_bounds__(NT, plane_min_blocks<T>(NT, RX1 * RX2, false, MANY))
 k_inv_xy(LocalPlan p, int band0, const C2<double>* __restrict__ psi, long long ldpsi,
          const int* __restrict__ plane_start, const int* __restrict__ pw_idx,
          const int* __restrict__ pw_pos, const C2<T>* __restrict__ twx,
@@ -510,6 +521,7 @@ template <typename T, int R1, int R2, int CB> constexpr size_t smem_z_band() {
 // The inverse half of B for the density: rho(r) += sum_b occ_b |psi_b(r)|^2. Thread and memory layout of
 // k_z_band; the sum over the CTA's bands of a point stays in a register of the thread that owns its
 // line in the second pass. part: null = add to rho, else the band groups' own boxes (summed by the caller).
+// 128 bands on 96 x 96 x 96: 304 us, the general form with its sums in shared memory 743.
 template <int R1, int R2, int CB>
 __global__ void __launch_bounds__(CB * R2, (z_min_blocks<R2, CB>(128)))
 k_z_density(LocalPlan p, int nbc, int per, const double* __restrict__ occ, const C2<double>* __restrict__ twz,
@@ -583,9 +595,12 @@ k_z_density(LocalPlan p, int nbc, int per, const double* __restrict__ occ, const
 // The non-collinear z stage of one spinor per step: both components' columns are transformed, multiplied by
 // [[V1+V2, V3-iV4], [V3+iV4, V1-V2]] and transformed back. One thread per (component, line, column); the
 // four potential columns are staged once per CTA and serve its bands, the kept points of the next spinor
-// are loaded while this one is transformed. Up slabs at W, down slabs nbc slabs later.
+// are loaded while this one is transformed. Up slabs at W, down slabs nbc slabs later. Bound: latency of
+// the FP64 passes. 80 spinors on 40 x 40 x 40, FP64: 84 us in 168 registers (three CTAs), 76 in 128 (four);
+// the general form that transforms one spinor per CTA through shared memory 495. Lines above 64 points hold
+// more and would spill in 128.
 template <typename T, int R1, int R2, int CB>
-__global__ void __launch_bounds__(2 * CB * R2, (z_min_blocks<R2, 2 * CB>(sizeof(T) == 8 ? 168 : 96)))
+__global__ void __launch_bounds__(2 * CB * R2, (z_min_blocks<R2, 2 * CB>(sizeof(T) == 4 ? 96 : R1 * R2 <= 64 ? 128 : 168)))
 k_z_spinor_band(LocalPlan p, int nbc, int per, const T* __restrict__ vu, const T* __restrict__ vd,
                 const T* __restrict__ vr, const T* __restrict__ vi, const C2<T>* __restrict__ twz, C2<T>* __restrict__ W) {
   constexpr int N3 = R1 * R2, NT = 2 * CB * R2, Q = quarter(R1);
@@ -685,8 +700,8 @@ k_z_spinor_band(LocalPlan p, int nbc, int per, const T* __restrict__ vu, const T
 // ---------------------------------------------------------------------------
 // C: forward y + forward x + gather + kinetic, one CTA per (band, kept z-plane)
 // ---------------------------------------------------------------------------
-template <typename T, int RX1, int RX2, int RY1, int RY2, int TC, bool PR, int NT = kThreadsPlanes>
-__global__ void __launch_bounds__(NT, plane_min_blocks<T>(NT, RX1 * RX2))
+template <typename T, int RX1, int RX2, int RY1, int RY2, int TC, bool PR, int NT = kThreadsPlanes, bool MANY = false>
+__global__ void __launch_bounds__(NT, plane_min_blocks<T>(NT, RX1 * RX2, true, MANY))
 k_fwd_xy(LocalPlan p, int band0, const C2<double>* __restrict__ psi, long long ldpsi,
          C2<double>* __restrict__ hpsi, long long ldh, const int* __restrict__ plane_start,
          const int* __restrict__ pw_idx, const int* __restrict__ pw_pos,
@@ -720,6 +735,15 @@ k_fwd_xy(LocalPlan p, int band0, const C2<double>* __restrict__ psi, long long l
   }
   const int e0 = plane_start[zi], e1 = plane_start[zi + 1];
 
+  // FP64 planes of up to 64 points: each thread's first point of the final gather (often the only one) is
+  // read ahead, its index here, psi and the kinetic term between the y and x transforms
+  constexpr bool kFirst = sizeof(T) == 8 && RX1 > 0 && RX1 * RX2 <= 64;
+  const bool first = kFirst && e0 + tid < e1;
+  int fi = 0, fp = 0;
+  if (first) {
+    fi = pw_idx[e0 + tid];
+    fp = pw_pos[e0 + tid];
+  }
   const C2<T>* Wp = W + ((size_t)b * p.nz + zi) * (size_t)p.plane;
   if (tid == 0 && p.plane * sizeof(C2<T>) % 16 == 0) {
     // bring the plane into L2 while the first tiles are transformed
@@ -767,7 +791,7 @@ k_fwd_xy(LocalPlan p, int band0, const C2<double>* __restrict__ psi, long long l
         });
       }
     }
-    if (sizeof(T) == 8 && xb == 0 && ekpg) {
+    if (sizeof(T) == 8 && !kFirst && xb == 0 && ekpg) {
       // bring the psi values and kinetic terms of the final gather into L2, so that its dependent
       // loads do not wait on HBM at the end of the CTA (FP64 only: in FP32 the extra registers cost a
       // CTA per SM on 96-point lines)
@@ -810,6 +834,12 @@ k_fwd_xy(LocalPlan p, int band0, const C2<double>* __restrict__ psi, long long l
     __syncthreads();
   }
 
+  C2<double> fs = czero<double>();
+  double fe = 0.0;
+  if (first && ekpg) {
+    fs = ps[fi];
+    fe = ekpg[fi];
+  }
   // forward x on the kept rows (row index fastest across lanes). The points lie in the slab's storage
   // order: slot(x) is where natural index x is (run-time radices: from a table in the tile buffer, which
   // is free by now and at least n1 shorts long: two rows of 32 columns, or more rows).
@@ -860,14 +890,15 @@ k_fwd_xy(LocalPlan p, int band0, const C2<double>* __restrict__ psi, long long l
 
   // gather the sphere and add the kinetic diagonal
   for (int e = e0 + tid; e < e1; e += nt) {
-    const int pos = pw_pos[e];
+    const bool f = kFirst && e == e0 + tid;
+    const int pos = f ? fp : pw_pos[e];
     const int x = pos & 0xffff, q = x / r1x;
     const C2<T> v = R[(size_t)(pos >> 16) * rowp + slot(r2x * (x - q * r1x) + q)];
-    const int i = pw_idx[e];
+    const int i = f ? fi : pw_idx[e];
     C2<double> out = mk<double>(double(v.x), double(v.y));
     if (ekpg) {
-      const C2<double> s = ps[i];
-      const double ek = ekpg[i];
+      const C2<double> s = f ? fs : ps[i];
+      const double ek = f ? fe : ekpg[i];
       out.x += ek * s.x;
       out.y += ek * s.y;
     }
@@ -880,22 +911,21 @@ k_fwd_xy(LocalPlan p, int band0, const C2<double>* __restrict__ psi, long long l
   }
 }
 
-// Threads of kernels A and C: one per line of the larger y pass; C keeps 256 where 384 measured slower
-// (FP32 on 96-point lines: 189 against 176 us for 160 bands).
-template <int RY1, int RY2, int TC> constexpr int threads_a() { return TC && RY1 ? TC * RY2 : kThreadsPlanes; }
-template <typename T, int RY1, int RY2, int TC> constexpr int threads_c() {
-  return sizeof(T) == 4 && RY1 * RY2 == 96 ? kThreadsPlanes : threads_a<RY1, RY2, TC>();
-}
+// Threads of kernels A and C: one per line of the larger y pass.
+template <int RY1, int RY2, int TC> constexpr int plane_threads() { return TC && RY1 ? TC * RY2 : kThreadsPlanes; }
 
 // Launch kernel A alone (scatter + inverse x + inverse y into the slab W).
 template <typename T, int RX1, int RX2, int RY1, int RY2, int TC>
 cudaError_t launch_a_impl(const LocalPlan& p, int nbc, int band0, const C2<double>* psi, long long ldpsi,
                           const int* plane_start, const int* pw_idx, const int* pw_pos, const C2<T>* twx,
                           const C2<T>* twy, C2<T>* W, cudaStream_t st) {
-  constexpr int NT = threads_a<RY1, RY2, TC>();
+  constexpr int NT = plane_threads<RY1, RY2, TC>();
   const size_t sm = smem_planes<T>(p);
   const bool pr = in_quarters(p.kd1, p.dx.r1, p.dx.r2) && in_quarters(p.kd2, p.dy.r1, p.dy.r2);
   auto* k = pr ? k_inv_xy<T, RX1, RX2, RY1, RY2, TC, true, NT> : k_inv_xy<T, RX1, RX2, RY1, RY2, TC, false, NT>;
+  if constexpr (RX1 == 0 && sizeof(T) == 4)
+    if (sm <= kManyPlaneBytes)
+      k = pr ? k_inv_xy<T, RX1, RX2, RY1, RY2, TC, true, NT, true> : k_inv_xy<T, RX1, RX2, RY1, RY2, TC, false, NT, true>;
   cudaError_t e = smem_limit((const void*)k, sm);
   if (e != cudaSuccess) return e;
   k<<<dim3(p.nz, nbc), NT, sm, st>>>(p, band0, psi, ldpsi, plane_start, pw_idx, pw_pos, twx, twy, W);
@@ -908,10 +938,13 @@ cudaError_t launch_c_impl(const LocalPlan& p, int nbc, int band0, const C2<doubl
                           C2<double>* hpsi, long long ldh, const int* plane_start, const int* pw_idx,
                           const int* pw_pos, const double* ekpg, const C2<T>* twx, const C2<T>* twy, const C2<T>* W,
                           cudaStream_t st) {
-  constexpr int NT = threads_c<T, RY1, RY2, TC>();
+  constexpr int NT = plane_threads<RY1, RY2, TC>();
   const size_t sm = smem_planes<T>(p);
   const bool pr = in_quarters(p.kd1, p.dx.r2, p.dx.r1) && in_quarters(p.kd2, p.dy.r2, p.dy.r1);
   auto* k = pr ? k_fwd_xy<T, RX1, RX2, RY1, RY2, TC, true, NT> : k_fwd_xy<T, RX1, RX2, RY1, RY2, TC, false, NT>;
+  if constexpr (RX1 == 0 && sizeof(T) == 4)
+    if (sm <= kManyPlaneBytes)
+      k = pr ? k_fwd_xy<T, RX1, RX2, RY1, RY2, TC, true, NT, true> : k_fwd_xy<T, RX1, RX2, RY1, RY2, TC, false, NT, true>;
   cudaError_t e = smem_limit((const void*)k, sm);
   if (e != cudaSuccess) return e;
   k<<<dim3(p.nz, nbc), NT, sm, st>>>(p, band0, psi, ldpsi, hpsi, ldh, plane_start, pw_idx, pw_pos, ekpg, twx, twy, W);
