@@ -329,6 +329,10 @@ static bool crt_ready(cpw_b200_ctx* c, int nb, cudaStream_t st) {
   return true;
 }
 
+bool ctx_residues(cpw_b200_ctx* c, int nb, cudaStream_t st) {
+  return c->nanl > 0 && c->nl_slices == 0 && crt_pays(c, nb) && crt_ready(c, nb, st);
+}
+
 int ctx_hkpsi_device(cpw_b200_ctx* c, int nb, const void* psi, long long ldpsi, void* hpsi, long long ldh,
                      cudaStream_t st, bool with_kinetic, bool with_nl) {
   if (!c->have_basis || !c->have_pot) return fail(kNotReady, "hk_psi: basis and potential must be set");

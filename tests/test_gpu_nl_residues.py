@@ -101,3 +101,20 @@ def test_new_projectors_and_precision_replace_the_planes(cuda):
     ref = _exact(x2, xnl2, psi)
     assert float(np.abs(_apply(cuda, ctx, psi) - ref).max() / np.abs(ref).max()) < TOL[H.FP64]
     ctx.close()
+
+
+@pytest.mark.parametrize("nb", [15, 40, 97])
+def test_drop_in_chunks(cuda, nb):
+    """The drop-in's band chunks (one; three and six of unequal size) with residue products, and again with
+    other projectors and waves, against the oracle (1e-12, the drop-in's tolerance)."""
+    from oracle import hk_psi as O
+    d = _basis("si2")
+    m = d["mtxd"]
+    for seed, na in ((nb, 20), (nb + 1, 33)):
+        x, xnl, _ = _random(m, na, 1, seed)
+        psi = configs.random_psi(m, nb, seed)
+        hpsi = np.zeros((m, nb), dtype=np.complex128, order="F")
+        H.hk_psi_c16(m, nb, psi, hpsi, False, d["ng"], np.asfortranarray(d["kgv"]), d["ekpg"], d["isort"], d["vscr"],
+                     d["kmscr"], x, xnl, na, m, nb, na, d["ng"], d["vscr"].size)
+        ref = O.hk_psi_c16(m, nb, psi, d["ekpg"], d["isort"], d["vscr"], d["kmscr"], d["kgv"], x, xnl)
+        assert np.abs(hpsi - ref).max() < 1e-12 * np.abs(ref).max()
