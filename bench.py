@@ -672,12 +672,12 @@ def run_ours(args, world, rank, local, dist):
                         for k, v in st64.items() if v[1]},
         "mixed": {"value": world * NB / (msmx / 1e3), "ms_per_step": msmx,
                   "speedup_vs_fp64": ms64 / msmx,
-                  "precision": "FP32 pruned FFT + V_loc, FP64 projector GEMMs",
+                  "precision": "FP32 pruned FFT + V_loc, FP64-accurate projector products (15 moduli)",
                   "stages": {k: v[0] / args.steps for k, v in stmx.items() if v[1]}},
         "mixed_tc": {"value": world * NB / (mstc / 1e3), "ms_per_step": mstc,
                      "speedup_vs_fp64": ms64 / mstc,
-                     "precision": "FP32 pruned FFT + V_loc, split-TF32 tcgen05 projector GEMMs "
-                                  "(hi.hi + hi.lo + lo.hi, FP64 drain of short FP32 chains)",
+                     "precision": "FP32 pruned FFT + V_loc, projector products as residue GEMMs on the int8 "
+                                  "tensor cores (9 moduli)",
                      "stages": {k: v[0] / args.steps for k, v in sttc.items() if v[1]},
                      "roofline": rooftc},
         "fp64_i8_projectors": {
@@ -686,8 +686,11 @@ def run_ours(args, world, rank, local, dist):
             "precision": "FP64 pruned FFT + V_loc, projector products in the FP64-accurate int8 tensor-core "
                          "Ozaki GEMM (7 slices; cpw_b200_set_projector_slices)",
             "stages": {k: v[0] / args.steps for k, v in results["fp64_i8"][1].items() if v[1]}},
-        "gpu_launches": int(sum(v[1] for k, v in st64.items() if k in ("inv_xy", "z_vloc", "fwd_xy"))),
-        "library_launches": {"cublas_zgemm": int(st64["nl_proj"][1] + st64["nl_expand"][1])},
+        # the residue form of one call's projector products is seven kernels (csrc/crt.cu)
+        "gpu_launches": int(sum(v[1] for k, v in st64.items() if k in ("inv_xy", "z_vloc", "fwd_xy"))
+                            + (7 * st64["nl_proj"][1] if os.environ.get("CPW_B200_NL_CRT") != "0" else 0)),
+        "library_launches": {"cublas_zgemm": int(st64["nl_proj"][1] + st64["nl_expand"][1])
+                             if os.environ.get("CPW_B200_NL_CRT") == "0" else 0},
         "clocks": clocks,
     }
     line["si64"] = si64_throughput(local, max(3, args.steps // 2), 3)
