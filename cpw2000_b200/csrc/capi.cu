@@ -114,8 +114,11 @@ struct DropinPipe {
   std::vector<int> start;     // band boundaries of the chunks (nchunk + 1)
 };
 
-int dropin_stage_in(cpw_b200_ctx* c, int m, int nb, const double* psi, long long ldh_host, DropinPipe* pp) {
-  int kChunks = 6;
+int dropin_stage_in(cpw_b200_ctx* c, int m, int nb, int nanl, const double* psi, long long ldh_host, DropinPipe* pp) {
+  // Four chunks where even their half-size ends (nb / 6 bands) pay for residue GEMMs, which read the X planes
+  // once per chunk: 480 bands of Si216 28.6 ms in six chunks, 26.8 in four. Else six (Si64's 160 bands, ZGEMMs
+  // beside the local kernels: 4 and 6 within the spread).
+  int kChunks = c->precision != 2 && c->nl_slices == 0 && residues_pay(c->precision, m, nanl, nb / 6) ? 4 : 6;
   constexpr int kMinChunk = 16;
   if (const char* v = getenv("CPW_B200_DROPIN_CHUNKS")) kChunks = std::max(1, atoi(v));
   DropinPipe& p = *pp;
@@ -712,7 +715,7 @@ int cpw_b200_hk_psi_c16(const int* mtxd, const int* neig, const double* psi, dou
   if (go) {
     const size_t bytes = (size_t)m * nb * 16;
     if ((s = c->h_in.ensure(bytes)) || (s = c->h_out.ensure(bytes)) ||
-        (s = dropin_stage_in(c, m, nb, psi, *mxddim, &pipe))) {
+        (s = dropin_stage_in(c, m, nb, *nanl, psi, *mxddim, &pipe))) {
       dropin_abandon(c);
       return s;
     }

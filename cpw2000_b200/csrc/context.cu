@@ -298,12 +298,15 @@ static int blas_fail(cublasStatus_t st, const char* what) {
 // waves, 864 projectors, 480 bands), 548 -> 394 (26,529, 256, 160), 119 -> 167 (18,577, 180, 37);
 // split TF32 5,900 -> 3,110, 303 -> 278, 98 -> 115 on the same three. CPW_B200_NL_CRT=1 / 0 forces
 // either way.
-static bool crt_pays(const cpw_b200_ctx* c, int nb) {
+bool residues_pay(int precision, int m, int nanl, int nb) {
   // int32 sums, a grid dimension, 16-bit sums over the K splits
-  if (c->nanl > kCrtMaxProjectors || nb > 65535 || c->mtxd > 15000000 || c->crt_off) return false;
+  if (nanl <= 0 || nanl > kCrtMaxProjectors || nb > 65535 || m > 15000000) return false;
   if (const char* v = getenv("CPW_B200_NL_CRT")) return atoi(v) != 0;
-  const double flops = 16.0 * c->mtxd * c->nanl * nb;
-  return c->precision == 2 ? nb >= 128 && flops >= 1.5e10 : nb >= 64 && flops >= 1e10;
+  const double flops = 16.0 * m * nanl * nb;
+  return precision == 2 ? nb >= 128 && flops >= 1.5e10 : nb >= 64 && flops >= 1e10;
+}
+static bool crt_pays(const cpw_b200_ctx* c, int nb) {
+  return !c->crt_off && residues_pay(c->precision, c->mtxd, c->nanl, nb);
 }
 
 // The residue GEMMs ready for nb bands: X converted, buffers allocated. Where memory does not suffice, or

@@ -263,7 +263,9 @@ int hamilt_kb_device(cpw_b200_ctx* c, int mtxd, const double* hdiag, const int* 
                      const double* delqnl, const double* vkb, const int* nkb, int ntype, const double* adot,
                      void* hamk, long long ldh, int mxdtyp, int mxdgve, int mxdnst, int mxdcub, int mxdlqp,
                      int mxddim);
-// whether ctx_hkpsi_device takes the residue GEMMs for nb bands; readies them if so
+// whether residue GEMMs are the better form of these projector products; whether ctx_hkpsi_device takes
+// them for nb bands (and readies them if so)
+bool residues_pay(int precision, int m, int nanl, int nb);
 bool ctx_residues(cpw_b200_ctx* c, int nb, cudaStream_t st);
 int ctx_hkpsi_device(cpw_b200_ctx* c, int nb, const void* psi, long long ldpsi, void* hpsi, long long ldh,
                      cudaStream_t st, bool with_kinetic, bool with_nl);
