@@ -273,6 +273,12 @@ __global__ void __launch_bounds__(256) k_mgs(MgsArgs a) {
 // nvec (nvec + 1) / 2 sums, each two shuffle trees and one trip between SMs. An mbarrier wait is limited
 // like the grid barrier's (polls); every CTA, also one that gave up, ends in the cluster barrier, so none
 // leaves while another may still store to its shared memory.
+//
+// Two sets of slots by the parity of the round are enough because every reader arrives: a store of round
+// r + 2 follows a collect of round r + 1, which waits for all gridDim.x * V blocks' arrivals of that round,
+// and a block arrives only behind its own barrier in post, which its warps reach after they have read the
+// slots of round r. The blocks of the last CTA that have no rows (the block count need be no multiple of V)
+// read the sums too, since they have to take the same branches: they arrive like the others, without a store.
 constexpr int kMgsRows = 512, kMgsCtas = 8, kMgsBlocks = 4;
 
 __device__ __forceinline__ void cluster_sync() {
@@ -304,7 +310,7 @@ template <int V> __global__ void __launch_bounds__(256 * V) k_mgs_cluster(MgsArg
   if (threadIdx.x == 0) {
     for (int p = 0; p < 2; ++p)
       asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"((unsigned)__cvta_generic_to_shared(&bar[p])),
-                   "r"(blocks)
+                   "r"(gridDim.x * V)
                    : "memory");
     asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   }
@@ -321,7 +327,7 @@ template <int V> __global__ void __launch_bounds__(256 * V) k_mgs_cluster(MgsArg
     }
     if (V == 1) __syncthreads();
     else asm volatile("bar.sync %0, 256;\n" ::"r"(vb + 1) : "memory");   // the block's own barrier
-    if (w == 0 && blk < blocks) {
+    if (w == 0) {
       double tot[3];
       for (int t = 0; t < k; ++t) {
         double s = lane < 8 ? sh[vb][t][lane] : 0.0;
@@ -329,9 +335,11 @@ template <int V> __global__ void __launch_bounds__(256 * V) k_mgs_cluster(MgsArg
         tot[t] = __shfl_sync(0xffffffffu, s, 0);
       }
       if (lane < gridDim.x) {
-        const unsigned dst = peer_address(&slot[par][blk][0], lane);
-        for (int t = 0; t < k; ++t)
-          asm volatile("st.shared::cluster.f64 [%0], %1;\n" ::"r"(dst + 8 * t), "d"(tot[t]) : "memory");
+        if (blk < blocks) {
+          const unsigned dst = peer_address(&slot[par][blk][0], lane);
+          for (int t = 0; t < k; ++t)
+            asm volatile("st.shared::cluster.f64 [%0], %1;\n" ::"r"(dst + 8 * t), "d"(tot[t]) : "memory");
+        }
         asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];\n" ::"r"(peer_address(&bar[par], lane))
                      : "memory");
       }

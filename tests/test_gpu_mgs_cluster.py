@@ -1,7 +1,8 @@
 """Modified Gram-Schmidt by one cluster against the grid form it replaces.
 
 Row counts at the edges of the rule (one block, two, the largest of each number of blocks to a CTA, the
-first that goes back to the grid), plane waves sorted by kinetic energy in a random potential. Both forms
+first that goes back to the grid) and block counts that leave one, two or three blocks of the last CTA
+without rows (9, 11, 13, 15 of 512 rows at two to a CTA; 17, 18, 19, 23, 30 at four), plane waves sorted by kinetic energy in a random potential. Both forms
 add the same parts in the same order, so whole eigensolves agree bit for bit; the vectors are orthonormal
 to rounding of sums of 16,385 products (1e-12).
 """
@@ -31,7 +32,8 @@ def _case(m):
     return d
 
 
-@pytest.mark.parametrize("m", [512, 513, 1024, 1025, 4096, 4097, 8192, 8193, 16384, 16385])
+@pytest.mark.parametrize("m", [512, 513, 1024, 1025, 4096, 4097, 8192, 8193, 16384, 16385,
+                               5600, 6600, 7680, 9100, 9700, 11700, 15300])
 def test_cluster_and_grid_forms_agree(cuda, m, monkeypatch):
     import torch
     d, nb = _case(m), 12
