@@ -1,4 +1,4 @@
-// PTX helpers of the tensor-core GEMM kernels (oz.cu, crt.cu): shared-memory operand descriptors,
+// PTX helpers of the tensor-core GEMM kernels (oz.cu, crt.cu, nl_tc.cu): shared-memory operand descriptors,
 // kind::i8 products, bounded mbarrier waits, bulk copies and tensor-memory reads.
 #pragma once
 #include <cuda_runtime.h>
@@ -14,11 +14,11 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)_
 // K-major operand tile, 128-byte swizzle: 8-row groups 1024 bytes apart
 __device__ __forceinline__ uint64_t smem_desc(uint32_t addr) {
   uint64_t d = 0;
-  d |= (uint64_t)((addr >> 4) & 0x3FFF);
-  d |= (uint64_t)1 << 16;
-  d |= (uint64_t)((1024 >> 4) & 0x3FFF) << 32;
-  d |= (uint64_t)1 << 46;
-  d |= (uint64_t)2 << 61;
+  d |= (uint64_t)((addr >> 4) & 0x3FFF);               // start address
+  d |= (uint64_t)1 << 16;                               // leading byte offset (unused for swizzled K-major)
+  d |= (uint64_t)((1024 >> 4) & 0x3FFF) << 32;          // stride byte offset: 8 rows x 128 B
+  d |= (uint64_t)1 << 46;                               // descriptor version
+  d |= (uint64_t)2 << 61;                               // 128-byte swizzle
   return d;
 }
 
@@ -58,7 +58,10 @@ __device__ __forceinline__ unsigned long long globaltimer_ns() {
   return t;
 }
 
-// wait bounded in time (limit_ns); gives up early once another role has recorded a failure
+// wait bounded in time (limit_ns); gives up early once another role has recorded a failure.
+// The hand-offs between the roles use the caller's limit (GemmArgs::wait_ns, 2 s unless a
+// failure-detection test shortens it); the waits for copies and MMAs already issued, before the
+// CTA exits, always use kWaitNs: those complete on their own.
 __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, const volatile int* failed,
                                           unsigned long long limit_ns = kWaitNs) {
   // a phase that is already complete costs no read of the timer (about a microsecond)
