@@ -236,10 +236,10 @@ __global__ void __launch_bounds__(kThreads, 1) k_crt_gemm(const __grid_constant_
     const uint32_t lane_base = tmem + ((uint32_t)(32 * quarter) << 16);
     const int ncol = g.nt / 2;                // columns of this warp's half: a multiple of 8
     int nit = 0;
-    for (int it = blockIdx.x; it < nitems && !failed; it += gridDim.x, ++nit) {
+    for (int it = blockIdx.x; it < nitems; it += gridDim.x, ++nit) {
       const Item w = item_of(g, it);
       const int buf = nit & 1;
-      if (!mbar_wait(smem_u32(&accf[buf]), (uint32_t)((nit / 2) & 1), &failed, g.wait_ns)) {
+      if (!mbar_wait_warp(smem_u32(&accf[buf]), (uint32_t)((nit / 2) & 1), &failed, g.wait_ns)) {
         failed = 1;
         atomicExch(g.err, 1);
         break;

@@ -76,6 +76,13 @@ __device__ __forceinline__ bool mbar_wait(uint32_t mbar, uint32_t parity, const 
   }
 }
 
+// The same for all lanes of a converged warp, with one answer: a lane that gave up alone would leave the others
+// to run the warp-wide tensor-memory loads without it.
+__device__ __forceinline__ bool mbar_wait_warp(uint32_t mbar, uint32_t parity, const volatile int* failed,
+                                               unsigned long long limit_ns) {
+  return __all_sync(0xffffffffu, mbar_wait(mbar, parity, failed, limit_ns));
+}
+
 __device__ __forceinline__ void mbar_init(uint32_t mbar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;\n" ::"r"(mbar), "r"(count));
 }

@@ -304,7 +304,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tf32x3(const GemmArgs g) {
     const int quarter = warp & 3, slice = (warp - 2) >> 2;
     const uint32_t lane_base = tmem + ((uint32_t)(32 * quarter) << 16);
     long long gq = 0;
-    for (int it = blockIdx.x; it < nitems && !failed; it += gridDim.x) {
+    for (int it = blockIdx.x; it < nitems; it += gridDim.x) {
       const Item w = item_of(g, it);
       const int nchunk = (w.nblk + chain - 1) / chain;
       double acc[kDrainCols];
@@ -313,7 +313,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tf32x3(const GemmArgs g) {
       bool ok = true;
       for (int q = 0; q < nchunk; ++q, ++gq) {
         const int b = (int)(gq % kMainBufs);
-        if (!mbar_wait(smem_u32(&accf[b]), (uint32_t)((gq / kMainBufs) & 1), &failed, g.wait_ns)) {
+        if (!mbar_wait_warp(smem_u32(&accf[b]), (uint32_t)((gq / kMainBufs) & 1), &failed, g.wait_ns)) {
           ok = false;
           failed = 1;
           atomicExch(g.err, 1);
@@ -340,7 +340,7 @@ __global__ void __launch_bounds__(kThreads, 1) k_gemm_tf32x3(const GemmArgs g) {
           if (lane == 0) mbar_arrive(smem_u32(pass == 0 ? &acce[b] : corre));
         }
       }
-      if (!ok || failed) break;
+      if (!ok) break;
 #define CPWB_ACC(j) (acc[j])
       const int m = w.m0 + 32 * quarter + lane;
       if (nchunk > 0 && w.m0 + 32 * quarter < g.M) {      // warp-uniform: the warp has valid rows

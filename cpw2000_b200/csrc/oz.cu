@@ -299,9 +299,9 @@ __global__ void __launch_bounds__(kThreads, 1) k_oz_gemm(const Args g) {
     const int quarter = warp & 3, half = (warp - 2) >> 2;
     const uint32_t lane_base = tmem + ((uint32_t)(32 * quarter) << 16);
     int nit = 0;
-    for (int it = blockIdx.x; it < nitems && !failed; it += gridDim.x, ++nit) {
+    for (int it = blockIdx.x; it < nitems; it += gridDim.x, ++nit) {
       const Item w = item_of(g, it);
-      if (!mbar_wait(smem_u32(accf), (uint32_t)(nit & 1), &failed, g.wait_ns)) {
+      if (!mbar_wait_warp(smem_u32(accf), (uint32_t)(nit & 1), &failed, g.wait_ns)) {
         failed = 1;
         atomicExch(g.err, 1);
         break;

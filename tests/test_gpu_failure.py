@@ -50,6 +50,42 @@ def test_mbarrier_wait_runs_out_and_context_recovers(cuda):
     ctx.close()
 
 
+@pytest.mark.parametrize("form", ["residues", "residues, 9 moduli", "split TF32", "int8 slices"])
+def test_gemm_roles_with_no_time_to_wait(cuda, form, monkeypatch):
+    """With a limit of 0 ns a role that has to wait at all may give up: the call then reports the time-out, and
+    the next one on the same context is right. Blocks of several tiles per CTA, so that every role waits."""
+    import torch
+    monkeypatch.setenv("CPW_B200_NL_CRT", "1" if "residues" in form else "0")
+    d = configs.kpoint_inputs(configs.si2_fcc(), 1)
+    rng = np.random.default_rng(3)
+    m, na, nb = d["mtxd"], 700, 300
+    x = np.asfortranarray(rng.standard_normal((m, na)) + 1j * rng.standard_normal((m, na)))
+    xnl = rng.choice((-1.0, 1.0), na)
+    ctx = H.Context(0, precision=H.FP64 if _fp64(form) else H.MIXED_TC)
+    ctx.set_kpoint(m, d["isort"], d["kgv"], 0 * d["ekpg"], d["kmscr"])
+    ctx.set_potential(0 * d["vscr"])
+    ctx.set_projectors(x, xnl)
+    L = _lib.lib()
+    if form == "int8 slices":
+        assert L.cpw_b200_set_projector_slices(ctx.handle, 7) == 0
+    psi = rng.standard_normal((m, nb)) + 1j * rng.standard_normal((m, nb))
+    dev = torch.from_numpy(np.ascontiguousarray(psi.T)).to(cuda).t()
+    out = torch.zeros((nb, m), dtype=torch.complex128, device=cuda).t()
+    for limit in (0, -1, 0, 200, -1):           # -1: the default
+        L.cpw_b200_set_wait_limits(ctx.handle, limit, -1)
+        ctx.hk_psi(dev, out)
+        status = L.cpw_b200_synchronize(ctx.handle)
+        assert status in ((0, TIMEOUT) if limit >= 0 else (0,))
+        if limit < 0:
+            ref = x @ (xnl[:, None] * (x.conj().T @ psi))
+            assert np.abs(out.cpu().numpy() - ref).max() < (1e-12 if _fp64(form) else 2e-5) * np.abs(ref).max()
+    ctx.close()
+
+
+def _fp64(form):
+    return form in ("residues", "int8 slices")
+
+
 def test_selftest_rejects_limits_above_two_seconds(cuda):
     ctx = H.Context(0)
     L = _lib.lib()
