@@ -13,7 +13,6 @@
 #include "context.hpp"
 
 namespace cpwb {
-const char* last_error();
 }
 
 using namespace cpwb;

@@ -319,7 +319,7 @@ static bool crt_ready(cpw_b200_ctx* c, int nb, cudaStream_t st) {
   const bool have = c->crt.L == L && c->crt.m == c->mtxd && c->crt.na == c->nanl;
   if (!have && !free_run) return false;
   if ((!have && crt_prepare(c->crt, c->mtxd, c->nanl, L, c->anl.p, c->anld.p, st)) ||
-      crt_reserve(c->crts, c->crt, nb, free_run)) {
+      crt_reserve(c->crts, c->crt, nb, free_run) || (free_run ? tc_error_flag(c->tcs) != kOk : !c->tcs.err.p)) {
     if (free_run) {
       cudaGetLastError();
       c->crt.buf.release();
@@ -441,7 +441,7 @@ int ctx_hkpsi_device(cpw_b200_ctx* c, int nb, const void* psi, long long ldpsi, 
   if (crt_nl) {
     cudaEvent_t t0 = c->timer.on ? c->timer.take() : nullptr, t1 = c->timer.on ? c->timer.take() : nullptr;
     cudaEvent_t t2 = c->timer.on ? c->timer.take() : nullptr;
-    if ((s = crt_nl_apply(c->crts, c->crt, nb, psi, ldpsi, hpsi, ldh, c->tcs.wait_ns, st, t0, t1, t2))) return s;
+    if ((s = crt_nl_apply(c->crts, c->crt, nb, psi, ldpsi, hpsi, ldh, c->tcs, st, t0, t1, t2))) return s;
     c->timer.mark(kStNlProj, t0, t1);
     c->timer.mark(kStNlExpand, t1, t2);
     return kOk;

@@ -41,6 +41,7 @@ struct StageTimer {
 };
 
 void set_error(const std::string& msg);
+const char* last_error();
 int fail(int code, const std::string& msg);
 int cuda_fail(cudaError_t e, const char* what);
 
@@ -116,14 +117,12 @@ struct CrtOperands {
   int nkb1 = 0, nkb2 = 0, tiles1 = 0, tiles2 = 0;
 };
 struct CrtScratch {
-  DevBuf buf, err;
+  DevBuf buf;
 };
 int crt_prepare(CrtOperands& o, int m, int na, int L, const void* anl, const void* anld, cudaStream_t st);
 int crt_reserve(CrtScratch& t, const CrtOperands& o, int nb, bool may_allocate);
 int crt_nl_apply(CrtScratch& t, const CrtOperands& o, int nb, const void* psi, long long ldpsi, void* hpsi,
-                 long long ldh, unsigned long long wait_ns, cudaStream_t st, cudaEvent_t t0, cudaEvent_t t1,
-                 cudaEvent_t t2);
-int crt_read_error(CrtScratch& t);
+                 long long ldh, const TcScratch& tcs, cudaStream_t st, cudaEvent_t t0, cudaEvent_t t1, cudaEvent_t t2);
 int tc_error_flag(TcScratch& t);
 int tc_read_error(TcScratch& t);
 int tc_prepare_projectors(cpw_b200_ctx* c);

@@ -823,19 +823,14 @@ Layout layout_of(const CrtOperands& o, const Sizes& z, int nb) {
 int crt_reserve(CrtScratch& t, const CrtOperands& o, int nb, bool may_allocate) {
   using namespace crt;
   const size_t need = layout_of(o, sizes_of(o, nb, num_sms()), nb).total;
-  if (!may_allocate) return t.err.p && t.buf.p && t.buf.bytes >= need ? kOk : kNotReady;
-  if (int s = t.buf.ensure(need)) return s;
-  if (!t.err.p) {
-    if (int s = t.err.ensure(sizeof(int))) return s;
-    cudaError_t e = cudaMemset(t.err.p, 0, sizeof(int));
-    if (e != cudaSuccess) return cuda_fail(e, "crt error flag");
-  }
-  return kOk;
+  if (!may_allocate) return t.buf.p && t.buf.bytes >= need ? kOk : kNotReady;
+  return t.buf.ensure(need);
 }
 
-// hpsi += X D X^H psi; hpsi already holds the local part. After crt_reserve for nb bands.
+// hpsi += X D X^H psi; hpsi already holds the local part. After crt_reserve for nb bands. A wait that gives up
+// sets the error flag of tcs (made by tc_error_flag), which tc_check_error reports.
 int crt_nl_apply(CrtScratch& t, const CrtOperands& o, int nb, const void* psi, long long ldpsi, void* hpsi,
-                 long long ldh, unsigned long long wait_ns, cudaStream_t st, cudaEvent_t t0, cudaEvent_t t1,
+                 long long ldh, const TcScratch& tcs, cudaStream_t st, cudaEvent_t t0, cudaEvent_t t1,
                  cudaEvent_t t2) {
   using namespace crt;
   const int nsm = num_sms(), m = o.m, na = o.na, L = o.L;
@@ -863,8 +858,8 @@ int crt_nl_apply(CrtScratch& t, const CrtOperands& o, int nb, const void* psi, l
   g1.nsplit = z.nsplit;
   g1.L = L;
   g1.ldr = (long long)o.tiles1 * BM;
-  g1.err = (int*)t.err.p;
-  g1.wait_ns = wait_ns;
+  g1.err = (int*)tcs.err.p;
+  g1.wait_ns = tcs.wait_ns;
   GemmArgs g2 = g1;
   g2.a = o.a2;
   g2.b = b2;
@@ -893,16 +888,6 @@ int crt_nl_apply(CrtScratch& t, const CrtOperands& o, int nb, const void* psi, l
   });
   if (e == cudaSuccess) e = cudaGetLastError();
   return e == cudaSuccess ? kOk : cuda_fail(e, "projector products (residues)");
-}
-
-int crt_read_error(CrtScratch& t) {
-  if (!t.err.p) return kOk;
-  int h = 0;
-  cudaError_t e = cudaMemcpy(&h, t.err.p, sizeof(int), cudaMemcpyDeviceToHost);
-  if (e != cudaSuccess) return cuda_fail(e, "crt error flag");
-  if (!h) return kOk;
-  cudaMemset(t.err.p, 0, sizeof(int));
-  return fail(kTimeout, "projector products: an mbarrier wait gave up");
 }
 
 }  // namespace cpwb

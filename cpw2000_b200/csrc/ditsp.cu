@@ -1201,9 +1201,10 @@ struct Trim {
 // The driver. psi/hpsi: device complex128 (ldp >= mtxd), mxdbnd columns.
 // hamsm: host complex(8) (mxdsml, mxdsml) column-major (first mtxds used).
 // hdiag: host real(mtxd). ei: host real(mxdbnd).
-int ditsp_device(cpw_b200_ctx* c, int ipr, int* ifail, int icmax, int iguess, double epspsi, int* neig_io, int mtxds,
-                 void* psi, long long ldp, void* hpsi, const double* hamsm, int mxdsml, const double* hdiag,
-                 int mxdbnd, double* ei, long long* ihkpsum, cudaStream_t st, double* itlog, int itlog_rows) {
+static int ditsp_solve(cpw_b200_ctx* c, int ipr, int* ifail, int icmax, int iguess, double epspsi, int* neig_io,
+                       int mtxds, void* psi, long long ldp, void* hpsi, const double* hamsm, int mxdsml,
+                       const double* hdiag, int mxdbnd, double* ei, long long* ihkpsum, cudaStream_t st, double* itlog,
+                       int itlog_rows) {
   if (!c->have_basis || !c->have_pot) return fail(kNotReady, "ditsp_c16: basis and potential must be set");
   const int mtxd = c->mtxd;
   int neig = *neig_io;
@@ -1851,8 +1852,24 @@ int ditsp_device(cpw_b200_ctx* c, int ipr, int* ifail, int icmax, int iguess, do
     fflush(stdout);
   }
   if ((s = S.ck(cudaStreamSynchronize(st), "ditsp"))) return s;
-  if (S.basis_i8 && (s = oz_read_error(c->ozs))) return s;
   return lconv ? kOk : kNotConverged;
+}
+
+// A tensor-core kernel of H|psi> or of a basis product that gave up leaves its output incomplete, whatever the solve
+// made of it: the time-out is reported ahead of the solve's own status.
+int ditsp_device(cpw_b200_ctx* c, int ipr, int* ifail, int icmax, int iguess, double epspsi, int* neig_io, int mtxds,
+                 void* psi, long long ldp, void* hpsi, const double* hamsm, int mxdsml, const double* hdiag,
+                 int mxdbnd, double* ei, long long* ihkpsum, cudaStream_t st, double* itlog, int itlog_rows) {
+  const int s = ditsp_solve(c, ipr, ifail, icmax, iguess, epspsi, neig_io, mtxds, psi, ldp, hpsi, hamsm, mxdsml, hdiag,
+                            mxdbnd, ei, ihkpsum, st, itlog, itlog_rows);
+  if (s == kOk || s == kNotConverged) {
+    const int t = tc_check_error(c);
+    return t ? t : s;
+  }
+  const std::string why = last_error();
+  if (cudaStreamSynchronize(st) == cudaSuccess && tc_check_error(c) == kTimeout) return kTimeout;
+  set_error(why);
+  return s;
 }
 
 void ditsp_release(cpw_b200_ctx* c) {

@@ -546,12 +546,13 @@ int grid_for(long long work, int nsm) {
 
 }  // namespace
 
-// the sticky error flag of the tensor-core kernels: zeroed when allocated, read and cleared by
+// the sticky error flag of the tensor-core kernels (split TF32 and residues): zeroed when allocated, read and cleared by
 // tc_check_error (a bounded wait that gave up in any launch since the last check reports)
 int tc_error_flag(TcScratch& t) {
   if (t.err.p) return kOk;
   if (int s = t.err.ensure(sizeof(int))) return s;
   cudaError_t e = cudaMemset(t.err.p, 0, sizeof(int));
+  if (e == cudaSuccess) e = cudaStreamSynchronize(cudaStreamLegacy);     // before kernels of other streams set it
   return e == cudaSuccess ? kOk : cuda_fail(e, "tc error flag");
 }
 
@@ -769,8 +770,7 @@ int tc_zgemm_nn(cpw_b200_ctx* c, int m, int n, int kk, const void* a, long long 
 
 int tc_check_error(cpw_b200_ctx* c) {
   if (int s = tc_read_error(c->tcs)) return s;
-  if (int s = oz_read_error(c->ozs)) return s;
-  return crt_read_error(c->crts);
+  return oz_read_error(c->ozs);
 }
 
 namespace tc {

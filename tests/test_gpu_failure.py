@@ -14,6 +14,7 @@ hangs the GPU:
    gives up at its first poll, so the eigensolver call returns
    CPW_B200_TIMEOUT; with the default limit restored the same context solves
    to the dense eigenvalues.
+3. the projector products' roles with a limit of 0 ns, and the eigensolver's status after one gave up.
 """
 import numpy as np
 import pytest
@@ -84,6 +85,29 @@ def test_gemm_roles_with_no_time_to_wait(cuda, form, monkeypatch):
 
 def _fp64(form):
     return form in ("residues", "int8 slices")
+
+
+@pytest.mark.parametrize("prec", [H.FP64, H.MIXED_TC])
+def test_eigensolver_reports_a_wait_that_gave_up(cuda, prec, monkeypatch):
+    """A tensor-core kernel that gave up leaves H|psi> incomplete: the solve that used it does not return success.
+    The flag is that of the projector products; the self-test raises it as a product of the solve would."""
+    import torch
+    monkeypatch.setenv("CPW_B200_NL_CRT", "1")
+    d = configs.kpoint_inputs(configs.si2_fcc(), 0, with_hamsm=True)
+    nb, m = 8, d["mtxd"]
+    ctx = H.Context(0, precision=prec).setup(d)
+
+    def solve():
+        psi = torch.zeros((3 * nb, m), dtype=torch.complex128, device=cuda).t()
+        return E.eigensolve(ctx, psi, torch.zeros_like(psi), nb, d["mtxds"], d["hamsm"], d["hdiag"], epspsi=1e-5)
+
+    assert _lib.lib().cpw_b200_wait_selftest(ctx.handle, 1_000_000, None) == 0
+    with pytest.raises(CpwB200Error) as ei:
+        solve()
+    assert ei.value.status == TIMEOUT
+    assert solve()["converged"]             # the flag is cleared once reported
+    ctx.synchronize()
+    ctx.close()
 
 
 def test_selftest_rejects_limits_above_two_seconds(cuda):
