@@ -283,6 +283,7 @@ int ctx_set_projectors(cpw_b200_ctx* c, int nanl, const double* anlga, int ld, c
   projectors_changed(c);
   e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return cuda_fail(e, "set_projectors");
+  if ((s = residues_follow(c))) return s;
   if (c->precision == 2) return tc_prepare_projectors(c);
   return kOk;
 }
@@ -309,13 +310,25 @@ static bool crt_pays(const cpw_b200_ctx* c, int nb) {
   return !c->crt_off && residues_pay(c->precision, c->mtxd, c->nanl, nb);
 }
 
+static int residue_moduli(const cpw_b200_ctx* c) { return c->precision == 2 ? 9 : 15; }
+
+// A replayed graph reads the planes whatever has happened since its capture, as it reads anl and anld in the
+// other forms, which the setters rewrite in place. So projectors of a shape that a capture has used are
+// converted by the setter; others by the first call that wants them.
+int residues_follow(cpw_b200_ctx* c) {
+  const CrtOperands::Shape now{c->mtxd, c->nanl, residue_moduli(c)};
+  const auto& used = c->crt.captured;
+  if (std::find(used.begin(), used.end(), now) == used.end()) return kOk;
+  return crt_prepare(c->crt, now.m, now.na, now.L, c->anl.p, c->anld.p, c->stream);
+}
+
 // The residue GEMMs ready for nb bands: X converted, buffers allocated. Where memory does not suffice, or
 // a stream capture forbids the preparation, the products stay on the other path.
 static bool crt_ready(cpw_b200_ctx* c, int nb, cudaStream_t st) {
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
   const bool free_run = cap == cudaStreamCaptureStatusNone;
-  const int L = c->precision == 2 ? 9 : 15;
+  const int L = residue_moduli(c);
   const bool have = c->crt.L == L && c->crt.m == c->mtxd && c->crt.na == c->nanl;
   if (!have && !free_run) return false;
   if ((!have && crt_prepare(c->crt, c->mtxd, c->nanl, L, c->anl.p, c->anld.p, st)) ||
@@ -329,6 +342,9 @@ static bool crt_ready(cpw_b200_ctx* c, int nb, cudaStream_t st) {
     }
     return false;
   }
+  const CrtOperands::Shape now{c->mtxd, c->nanl, L};
+  auto& used = c->crt.captured;
+  if (!free_run && std::find(used.begin(), used.end(), now) == used.end()) used.push_back(now);
   return true;
 }
 

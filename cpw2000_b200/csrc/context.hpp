@@ -115,6 +115,11 @@ struct CrtOperands {
   int* s2 = nullptr;
   int m = 0, na = 0, L = 0;
   int nkb1 = 0, nkb2 = 0, tiles1 = 0, tiles2 = 0;
+  struct Shape {
+    int m, na, L;
+    bool operator==(const Shape& o) const { return m == o.m && na == o.na && L == o.L; }
+  };
+  std::vector<Shape> captured;      // shapes that a stream capture has used
 };
 struct CrtScratch {
   DevBuf buf;
@@ -266,6 +271,8 @@ int hamilt_kb_device(cpw_b200_ctx* c, int mtxd, const double* hdiag, const int* 
 // them for nb bands (and readies them if so)
 bool residues_pay(int precision, int m, int nanl, int nb);
 bool ctx_residues(cpw_b200_ctx* c, int nb, cudaStream_t st);
+// after new projectors: the planes that a captured call reads are re-made in place
+int residues_follow(cpw_b200_ctx* c);
 int ctx_hkpsi_device(cpw_b200_ctx* c, int nb, const void* psi, long long ldpsi, void* hpsi, long long ldh,
                      cudaStream_t st, bool with_kinetic, bool with_nl);
 }  // namespace cpwb

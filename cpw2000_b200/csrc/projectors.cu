@@ -407,6 +407,7 @@ int ctx_proj_nl_kb(cpw_b200_ctx* c, const double* rkpt, int ntype, const int* na
   // the small tables are freed at return: finish with them first
   e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return cuda_fail(e, "proj_nl_kb");
+  if (int s = residues_follow(c)) return s;
   if (c->precision == 2) return tc_prepare_projectors(c);
   return kOk;
 }

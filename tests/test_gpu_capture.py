@@ -1,0 +1,54 @@
+"""A captured H|psi> replayed after new projectors of the same shape equals the eager call with them.
+
+The default projector forms: FP64 ZGEMMs, split TF32 and residue products of both. Replay and eager call run the
+same kernels on the same data: equal to the bit. In between, projectors of another shape are set and used.
+"""
+import numpy as np
+import pytest
+
+from cpw2000_b200 import configs
+from cpw2000_b200 import hk_psi as H
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("prec,crt", [(H.FP64, "0"), (H.FP64, "1"), (H.MIXED_TC, "0"), (H.MIXED_TC, "1")])
+def test_replay_follows_the_projectors(cuda, prec, crt, monkeypatch):
+    import torch
+    monkeypatch.setenv("CPW_B200_NL_CRT", crt)
+    d = configs.kpoint_inputs(configs.si2_fcc(), 1)
+    m, na, nb = d["mtxd"], 150, 20
+    rng = np.random.default_rng(7)
+    sets = []
+    for n in (na, na, na + 9):
+        x = np.asfortranarray(rng.standard_normal((m, n)) + 1j * rng.standard_normal((m, n)))
+        sets.append((x, rng.choice((-1.0, 1.0), n)))
+    ctx = H.Context(0, precision=prec)
+    ctx.set_kpoint(m, d["isort"], d["kgv"], d["ekpg"], d["kmscr"])
+    ctx.set_potential(d["vscr"])
+    ctx.set_projectors(*sets[2])
+    psi = torch.randn((nb, m), dtype=torch.complex128, device=cuda).t()
+    out, eager = torch.zeros_like(psi), torch.zeros_like(psi)
+    ctx.hk_psi(psi, eager)                  # the largest buffers first
+    ctx.set_projectors(*sets[0])
+    ctx.hk_psi(psi, eager)
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ctx.hk_psi(psi, out)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, eager)
+    before = eager.clone()
+    ctx.set_projectors(*sets[2])            # another shape, used
+    ctx.hk_psi(psi, eager)
+    torch.cuda.synchronize()
+    ctx.set_projectors(*sets[1])            # the captured shape, other values: no eager call before the replay
+    graph.replay()
+    torch.cuda.synchronize()
+    ctx.hk_psi(psi, eager)
+    torch.cuda.synchronize()
+    assert not torch.equal(eager, before)
+    assert torch.equal(out, eager)
+    graph.reset()
+    ctx.close()
