@@ -319,7 +319,9 @@ int residues_follow(cpw_b200_ctx* c) {
   const CrtOperands::Shape now{c->mtxd, c->nanl, residue_moduli(c)};
   const auto& used = c->crt.captured;
   if (std::find(used.begin(), used.end(), now) == used.end()) return kOk;
-  return crt_prepare(c->crt, now.m, now.na, now.L, c->anl.p, c->anld.p, c->stream);
+  if (int s = crt_prepare(c->crt, now.m, now.na, now.L, c->anl.p, c->anld.p, c->stream)) return s;
+  const cudaError_t e = cudaStreamSynchronize(c->stream);       // as the rest of the setters' work
+  return e == cudaSuccess ? kOk : cuda_fail(e, "projector residues");
 }
 
 // The residue GEMMs ready for nb bands: X converted, buffers allocated. Where memory does not suffice, or

@@ -489,30 +489,37 @@ __global__ void __launch_bounds__(256) k_crt_conv_cols(int m, int ncol, const do
   residues8<L, DIFF>(re, im, [&](int lc, uint2 w) { *reinterpret_cast<uint2*>(o + lc * plane) = w; });
 }
 
-// Rows of a complex block (m x K, columns strided): row i of the X-side planes of the expansion. One
-// thread converts the 128 complex numbers of one K block of one row (coalesced over rows).
+// Rows of a complex block (m x K, columns strided): row i of the X-side planes of the expansion. One block
+// converts the 128 complex numbers of one K block of 16 rows, staged through shared memory: its loads are
+// 256 contiguous bytes per column and a warp stores two whole rows of a tile (a thread per row stored
+// pieces of 8 bytes that lie 128 apart).
 template <int L>
-__global__ void __launch_bounds__(128) k_crt_conv_rows(int m, int K, const double2* __restrict__ x, long long ldx,
+__global__ void __launch_bounds__(256) k_crt_conv_rows(int m, int K, const double2* __restrict__ x, long long ldx,
                                                        const int* __restrict__ s, int tiles, int nkb,
                                                        int8_t* __restrict__ out) {
-  const int i = blockIdx.x * 128 + threadIdx.x, kb = blockIdx.y;
+  constexpr int kRow = 16 * 9 + 1;        // a row's 16 pieces of 8 numbers, spread over the banks
+  __shared__ double2 buf[16 * kRow];
+  const int i0 = blockIdx.x * 16, kb = blockIdx.y, tid = threadIdx.x;
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const int t = tid + 256 * j, row = t & 15, k = t >> 4, kk = kb * KB + k;
+    buf[row * kRow + (k >> 3) * 9 + (k & 7)] =
+        i0 + row < m && kk < K ? x[(size_t)kk * ldx + i0 + row] : make_double2(0.0, 0.0);
+  }
+  __syncthreads();
+  const int row = tid >> 4, c = tid & 15, i = i0 + row;
   if (i >= m) return;
   const Scale f = scale_of(s[i]);
-  int8_t* o = out + ((size_t)(i / BM) * nkb + kb) * kATile;
-  const size_t plane = (size_t)tiles * nkb * kATile;
-  for (int c = 0; c < 16; ++c) {
-    Limbs re[8], im[8];
+  Limbs re[8], im[8];
 #pragma unroll
-    for (int u = 0; u < 8; ++u) {
-      const int k = kb * KB + c * 8 + u;
-      const double2 v = k < K ? x[(size_t)k * ldx + i] : make_double2(0.0, 0.0);
-      re[u] = limbs(v.x, f);
-      im[u] = limbs(v.y, f);
-    }
-    residues8<L, false>(re, im, [&](int lc, uint2 w) {
-      *reinterpret_cast<uint2*>(o + lc * plane + swz8(i % BM, c)) = w;
-    });
+  for (int u = 0; u < 8; ++u) {
+    const double2 v = buf[row * kRow + c * 9 + u];
+    re[u] = limbs(v.x, f);
+    im[u] = limbs(v.y, f);
   }
+  int8_t* o = out + ((size_t)(i / BM) * nkb + kb) * kATile + swz8(i % BM, c);
+  const size_t plane = (size_t)tiles * nkb * kATile;
+  residues8<L, false>(re, im, [&](int lc, uint2 w) { *reinterpret_cast<uint2*>(o + lc * plane) = w; });
 }
 
 // ------------------------------------------------------------------ residues to numbers
@@ -727,7 +734,8 @@ int num_sms() {
 
 }  // namespace crt
 
-// Convert X (anl, m x na, ld m) and X D (anld) once per projector set; the work is complete on return.
+// Convert X (anl, m x na, ld m) and X D (anld) once per projector set, on st: a call on another stream is ordered
+// behind it as behind any earlier call, whose slab and scratch it shares.
 int crt_prepare(CrtOperands& o, int m, int na, int L, const void* anl, const void* anld, cudaStream_t st) {
   using namespace crt;
   o.L = 0;
@@ -753,11 +761,10 @@ int crt_prepare(CrtOperands& o, int m, int na, int L, const void* anl, const voi
     constexpr int LL = decltype(lc)::value;
     k_crt_conv_cols<LL, true><<<dim3((o.nkb1 * KB + kConvPer - 1) / kConvPer, na), 256, 0, st>>>(
         m, na, (const double2*)anl, m, part, nchunk, pl.beta_a, BM, o.tiles1, o.nkb1, o.a1, o.s1);
-    k_crt_conv_rows<LL><<<dim3((m + 127) / 128, o.nkb2), 128, 0, st>>>(m, na, (const double2*)anld, m, o.s2,
-                                                                      o.tiles2, o.nkb2, o.a2);
+    k_crt_conv_rows<LL><<<dim3((m + 15) / 16, o.nkb2), 256, 0, st>>>(m, na, (const double2*)anld, m, o.s2, o.tiles2,
+                                                                     o.nkb2, o.a2);
   });
   cudaError_t e = cudaGetLastError();
-  if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return cuda_fail(e, "projector residues");
   o.m = m;
   o.na = na;
