@@ -218,6 +218,7 @@ int dropin_compute_out(cpw_b200_ctx* c, const DropinPipe& p, double* hpsi, bool 
       cuDoubleComplex* pk = (cuDoubleComplex*)c->proj.p + (size_t)b0 * c->nanl;
       if ((e = cudaStreamWaitEvent(c->s_nl, in_done, 0)) != cudaSuccess) return cuda_fail(e, "hk_psi_c16 pipeline");
       cublasSetStream(c->blas_nl, c->s_nl);
+      ++c->forms[kFormZgemm];
       // P_k = X^H psi_k (hk_psi_nl_c16.f90:82)
       if (cublasZgemm(c->blas_nl, CUBLAS_OP_C, CUBLAS_OP_N, c->nanl, nbc, m, &one, (const cuDoubleComplex*)c->anl.p, m,
                       (const cuDoubleComplex*)(din + (size_t)b0 * m), m, &zero, pk, c->nanl) != CUBLAS_STATUS_SUCCESS)
@@ -481,6 +482,14 @@ int cpw_b200_wait_selftest(cpw_b200_ctx* c, long long limit_ns, void* stream) {
   if (limit_ns < 0 || limit_ns > 2000000000LL) return fail(kBadArg, "wait_selftest: limit outside 0 .. 2 s");
   cudaSetDevice(c->device);
   return tc_wait_selftest(c, (unsigned long long)limit_ns, stream ? (cudaStream_t)stream : c->stream);
+}
+
+int cpw_b200_form_counts(cpw_b200_ctx* c, long long* counts, int n) {
+  if (!c) {
+    if (int s = default_ctx(&c)) return s;
+  }
+  for (int i = 0; i < n; ++i) counts[i] = i < kNumForms ? c->forms[i] : 0;
+  return kOk;
 }
 
 int cpw_b200_set_projector_slices(cpw_b200_ctx* c, int slices) {

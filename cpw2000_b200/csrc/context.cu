@@ -403,6 +403,7 @@ int ctx_hkpsi_device(cpw_b200_ctx* c, int nb, const void* psi, long long ldpsi, 
     ov_t1 = c->timer.on ? c->timer.take() : nullptr;
     if (ov_t0) cudaEventRecord(ov_t0, c->s_nl);
     cublasSetStream(c->blas_nl, c->s_nl);
+    ++c->forms[kFormZgemm];
     const cuDoubleComplex one = make_cuDoubleComplex(1.0, 0.0), zero = make_cuDoubleComplex(0.0, 0.0);
     // P = X^H psi (hk_psi_nl_c16.f90:82)
     if (cublasZgemm(c->blas_nl, CUBLAS_OP_C, CUBLAS_OP_N, c->nanl, nb, c->mtxd, &one, (const cuDoubleComplex*)c->anl.p,
@@ -459,6 +460,7 @@ int ctx_hkpsi_device(cpw_b200_ctx* c, int nb, const void* psi, long long ldpsi, 
   if (crt_nl) {
     cudaEvent_t t0 = c->timer.on ? c->timer.take() : nullptr, t1 = c->timer.on ? c->timer.take() : nullptr;
     cudaEvent_t t2 = c->timer.on ? c->timer.take() : nullptr;
+    ++c->forms[kFormResidues];
     if ((s = crt_nl_apply(c->crts, c->crt, nb, psi, ldpsi, hpsi, ldh, c->tcs, st, t0, t1, t2))) return s;
     c->timer.mark(kStNlProj, t0, t1);
     c->timer.mark(kStNlExpand, t1, t2);
@@ -480,6 +482,7 @@ int ctx_hkpsi_device(cpw_b200_ctx* c, int nb, const void* psi, long long ldpsi, 
           return s;
         c->oz_nl_ready = true;
       }
+      ++c->forms[kFormSlices];
       if (t0) cudaEventRecord(t0, st);
       // P = X^H psi (hk_psi_nl_c16.f90:82); hpsi += (X D) P (:87-96)
       if ((s = oz_gemm_prepared(c->ozs, c->oz_x, nb, psi, ldpsi, 1.0, false, c->proj.p, c->nanl, c->tcs.wait_ns, st)))
@@ -494,11 +497,13 @@ int ctx_hkpsi_device(cpw_b200_ctx* c, int nb, const void* psi, long long ldpsi, 
     }
     if (c->precision == 2 && c->tc_ready) {
       // opt-in mixed form: split-TF32 tensor-core products (nl_tc.cu)
+      ++c->forms[kFormSplitTf32];
       if ((s = tc_nl_apply(c, nb, psi, ldpsi, hpsi, ldh, st, t0, t1, t2))) return s;
       c->timer.mark(kStNlProj, t0, t1);
       c->timer.mark(kStNlExpand, t1, t2);
       return kOk;
     }
+    ++c->forms[kFormZgemm];
     if (t0) cudaEventRecord(t0, st);
     // P = X^H psi (hk_psi_nl_c16.f90:82); hpsi += (X D) P (:87-96)
     bs = cublasZgemm(c->blas, CUBLAS_OP_C, CUBLAS_OP_N, c->nanl, nb, c->mtxd, &one, (const cuDoubleComplex*)c->anl.p,

@@ -962,7 +962,10 @@ struct Solver {
     // allows: 4,096 rows 37 us, two blocks 49 at 4,700, four 82 at 9,000; the grid form 91, 101 and 139); the
     // grid form beyond, and for a block that one CTA holds, which waits for nobody. CPW_B200_MGS_GRID=1 keeps it.
     const char* gv = getenv("CPW_B200_MGS_GRID");
-    if (!(gv && atoi(gv) != 0) && grid > 1 && grid == (m + kMgsRows - 1) / kMgsRows && grid <= kMgsCtas * kMgsBlocks) {
+    const bool one_cluster = !(gv && atoi(gv) != 0) && grid > 1 && grid == (m + kMgsRows - 1) / kMgsRows &&
+                             grid <= kMgsCtas * kMgsBlocks;
+    ++c->forms[one_cluster ? kFormMgsCluster : kFormMgsGrid];
+    if (one_cluster) {
       const cudaError_t e = grid <= kMgsCtas       ? launch_mgs_cluster<1>(a, grid, st)
                             : grid <= 2 * kMgsCtas ? launch_mgs_cluster<2>(a, grid, st)
                                                    : launch_mgs_cluster<4>(a, grid, st);

@@ -156,6 +156,12 @@ class Context:
     def timing_begin(self):
         check(self._L.cpw_b200_timing_begin(self.handle))
 
+    FORMS = ("zgemm", "split_tf32", "residues", "slices", "mgs_cluster", "mgs_grid")
+
+    def form_counts(self) -> dict:
+        """Calls per form of the projector products and of the Gram-Schmidt leaves since the context was made."""
+        return form_counts(self.handle)
+
     def timing_end(self) -> dict:
         """Per-stage {name: (total_ms, launches)} since timing_begin (synchronises)."""
         ms = (C.c_double * 8)()
@@ -331,6 +337,13 @@ class Context:
         check(fn(self.handle, nb, C.c_void_p(psi.data_ptr()), self._ld(psi), C.c_void_p(hpsi.data_ptr()),
                  self._ld(hpsi), C.c_void_p(s)))
         return hpsi
+
+
+def form_counts(handle=None) -> dict:
+    """Calls per form (Context.FORMS) of a context, or of the drop-in entry points' own one."""
+    n = (C.c_longlong * len(Context.FORMS))()
+    check(_lib.lib().cpw_b200_form_counts(handle, n, len(Context.FORMS)))
+    return dict(zip(Context.FORMS, map(int, n)))
 
 
 def torch_stream_handle(device=None) -> int:

@@ -121,6 +121,12 @@ int cpw_b200_zgemm_i8_tri(cpw_b200_ctx* ctx, int transa, int m, int n, int k, co
                           const void* b, long long ldb, double alpha, int accumulate, void* c, long long ldc, int slices,
                           int tri, void* stream);
 
+/* How often each form that the library chooses between by size has been taken since the context was
+ * made (NULL: the context of the drop-in entry points), counted on the host per call: 0 cuBLAS ZGEMM,
+ * 1 split-TF32, 2 residue, 3 int8-slice projector products of H|psi>; 4 one-cluster, 5 grid form of the
+ * eigensolver's Gram-Schmidt leaves. */
+int cpw_b200_form_counts(cpw_b200_ctx* ctx, long long* counts, int n);
+
 /* Stage timers (CUDA events around each kernel of a stage, on the stream the
  * kernel runs on). timing_end synchronises and writes per-stage totals in ms
  * and launch counts for stages 0..nstage-1: 0 scatter+inverse xy, 1 inverse z +

@@ -44,8 +44,11 @@ def test_cluster_and_grid_forms_agree(cuda, m, monkeypatch):
     for grid in ("0", "1"):
         monkeypatch.setenv("CPW_B200_MGS_GRID", grid)
         psi = torch.zeros((3 * nb, m), dtype=torch.complex128, device=cuda).t()
+        before = ctx.form_counts()
         r = E.eigensolve(ctx, psi, torch.zeros_like(psi), nb, 60, d["hamsm"], d["ekpg"] + d["vscr"].mean(), epspsi=1e-5)
         assert r["converged"]
+        ran = {k for k, n in ctx.form_counts().items() if k.startswith("mgs") and n != before[k]}
+        assert ran == {"mgs_cluster" if grid == "0" and 512 < m <= 16384 else "mgs_grid"}
         p = psi[:, :nb].cpu().numpy()
         assert np.abs(p.conj().T @ p - np.eye(nb)).max() < 1e-12
         out.append((r["ei"], p))

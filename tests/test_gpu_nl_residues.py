@@ -37,8 +37,10 @@ def _apply(cuda, ctx, psi):
     # strides given outright: a transposed single column may report any
     p, h = (torch.empty_strided(psi.shape, (1, psi.shape[0]), dtype=torch.complex128, device=cuda) for _ in range(2))
     p.copy_(torch.from_numpy(psi))
+    before = ctx.form_counts()
     ctx.hk_psi(p, h)
     ctx.synchronize()
+    assert {k: n - before[k] for k, n in ctx.form_counts().items() if n != before[k]} == {"residues": 1}
     return h.cpu().numpy()
 
 
@@ -95,18 +97,36 @@ def test_new_projectors_and_precision_replace_the_planes(cuda):
     d = _basis("si2")
     x, xnl, psi = _random(d["mtxd"], 20, 6, 7)
     x2, xnl2, _ = _random(d["mtxd"], 31, 6, 8)
-    ctx = _context(d, H.FP64, x, xnl)
+    x3, xnl3, _ = _random(d["mtxd"], 31, 6, 9)
+    ctx = _context(d, H.MIXED, x, xnl)
     _apply(cuda, ctx, psi)
     ctx.set_projectors(x2, xnl2)
     ref = _exact(x2, xnl2, psi)
-    assert float(np.abs(_apply(cuda, ctx, psi) - ref).max() / np.abs(ref).max()) < TOL[H.FP64]
+    assert float(np.abs(_apply(cuda, ctx, psi) - ref).max() / np.abs(ref).max()) < TOL[H.MIXED]
+    ctx.set_precision(H.MIXED_TC)         # 9 moduli on the same projectors, then 15 again
+    nine = _apply(cuda, ctx, psi)
+    assert float(np.abs(nine - ref).max() / np.abs(ref).max()) < TOL[H.MIXED_TC]
+    ctx.set_precision(H.MIXED)
+    fifteen = _apply(cuda, ctx, psi)
+    assert float(np.abs(fifteen - ref).max() / np.abs(ref).max()) < TOL[H.MIXED]
+    assert not np.array_equal(nine, fifteen)
+    ctx.set_projectors(x3, xnl3)          # the same shape
+    ref = _exact(x3, xnl3, psi)
+    assert float(np.abs(_apply(cuda, ctx, psi) - ref).max() / np.abs(ref).max()) < TOL[H.MIXED]
     ctx.close()
 
 
-@pytest.mark.parametrize("nb", [15, 40, 97])
-def test_drop_in_chunks(cuda, nb):
-    """The drop-in's band chunks (one; three and six of unequal size) with residue products, and again with
-    other projectors and waves, against the oracle (1e-12, the drop-in's tolerance)."""
+@pytest.mark.parametrize("nb,chunks", [(15, 1), (40, 3), (97, 4), (97, 6)])
+def test_drop_in_chunks(cuda, nb, chunks, monkeypatch):
+    """The drop-in's band chunks (one; three, four and six with half-size ends) with residue products, and again with
+    other projectors and waves, against the oracle (1e-12, the drop-in's tolerance). Residues everywhere take
+    four chunks by themselves."""
+    if chunks == 6:
+        monkeypatch.setenv("CPW_B200_DROPIN_CHUNKS", "6")
+    _drop_in(nb, lambda n: n == {"residues": chunks})
+
+
+def _drop_in(nb, forms):
     from oracle import hk_psi as O
     d = _basis("si2")
     m = d["mtxd"]
@@ -114,7 +134,33 @@ def test_drop_in_chunks(cuda, nb):
         x, xnl, _ = _random(m, na, 1, seed)
         psi = configs.random_psi(m, nb, seed)
         hpsi = np.zeros((m, nb), dtype=np.complex128, order="F")
+        before = H.form_counts()
         H.hk_psi_c16(m, nb, psi, hpsi, False, d["ng"], np.asfortranarray(d["kgv"]), d["ekpg"], d["isort"], d["vscr"],
                      d["kmscr"], x, xnl, na, m, nb, na, d["ng"], d["vscr"].size)
+        assert forms({k: n - before[k] for k, n in H.form_counts().items() if n != before[k]})
         ref = O.hk_psi_c16(m, nb, psi, d["ekpg"], d["isort"], d["vscr"], d["kmscr"], d["kgv"], x, xnl)
         assert np.abs(hpsi - ref).max() < 1e-12 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("prec", [H.FP64, H.MIXED_TC])
+def test_first_call_on_new_projectors_does_not_wait(cuda, prec):
+    """The conversion of new projectors is queued like the rest of the call: hk_psi returns while earlier work of
+    its stream still runs."""
+    import torch
+    d = _basis("si2")
+    x, xnl, psi = _random(d["mtxd"], 40, 6, 11)
+    ctx = _context(d, prec, x, xnl)
+    _apply(cuda, ctx, psi)                 # sizes the buffers
+    ctx.set_projectors(x[:, ::-1], xnl[::-1].copy())
+    p, h = (torch.zeros((6, d["mtxd"]), dtype=torch.complex128, device=cuda).t() for _ in range(2))
+    p.copy_(torch.from_numpy(psi))
+    torch.cuda.synchronize()
+    busy = torch.cuda.Event()
+    torch.cuda._sleep(10 ** 9)             # about half a second
+    busy.record()
+    ctx.hk_psi(p, h)
+    assert not busy.query()
+    ctx.synchronize()
+    ref = _exact(x, xnl, psi)
+    assert float(np.abs(h.cpu().numpy() - ref).max() / np.abs(ref).max()) < TOL[prec]
+    ctx.close()
