@@ -307,7 +307,9 @@ bool residues_pay(int precision, int m, int nanl, int nb) {
   return precision == 2 ? nb >= 128 && flops >= 1.5e10 : nb >= 64 && flops >= 1e10;
 }
 static bool crt_pays(const cpw_b200_ctx* c, int nb) {
-  return !c->crt_off && residues_pay(c->precision, c->mtxd, c->nanl, nb);
+  // a MIXED_TC solve keeps split TF32 for all its blocks (ditsp.cu)
+  if (c->crt_off || (c->solving && c->precision == 2 && !getenv("CPW_B200_NL_CRT"))) return false;
+  return residues_pay(c->precision, c->mtxd, c->nanl, nb);
 }
 
 static int residue_moduli(const cpw_b200_ctx* c) { return c->precision == 2 ? 9 : 15; }

@@ -200,6 +200,7 @@ struct cpw_b200_ctx {
   cpwb::CrtOperands crt;
   cpwb::CrtScratch crts;
   bool crt_off = false;
+  bool solving = false;         // inside ditsp_device
   long long tc_k1p = 0, tc_k2p = 0;     // K blocks (32 reals) of the projection and expansion operands
   bool tc_ready = false;
 
