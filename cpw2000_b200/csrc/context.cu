@@ -292,19 +292,36 @@ static int blas_fail(cublasStatus_t st, const char* what) {
   return fail(kCublas, std::string(what) + ": cuBLAS status " + std::to_string((int)st));
 }
 
-// Whether the projector products of nb bands run as residue GEMMs (crt.cu). Their cost is mostly the X
-// planes (90 bytes per element of X in FP64, 54 in MIXED_TC) until there are enough bands to share
-// them, plus conversions and five more launches than the two GEMMs they replace: ~110 us of fixed
-// cost. Measured both ways (us, other form -> residues): FP64 ZGEMMs 17,040 -> 4,630 (88,951 plane
-// waves, 864 projectors, 480 bands), 548 -> 394 (26,529, 256, 160), 119 -> 167 (18,577, 180, 37);
-// split TF32 5,900 -> 3,110, 303 -> 278, 98 -> 115 on the same three. CPW_B200_NL_CRT=1 / 0 forces
-// either way.
+// Whether the projector products of nb bands run as residue GEMMs (crt.cu). CPW_B200_NL_CRT=1 / 0 forces either
+// way.
+//
+// FP64 and MIXED, where the other form is a pair of ZGEMMs of the same accuracy: where the time saved over
+// kResidueCalls calls covers the conversion of X and X D, which the first call on new projectors makes (a solve
+// applies H ten times and more per projector set). In us, fitted to 40 measured shapes (9,898 to 89,137 plane
+// waves, 32 to 1,500 projectors, 4 to 480 bands): ZGEMMs at 33 TFLOP/s; residues 75 for their seven launches,
+// 15e-6 per element of X (its planes are read) and 55e-6 per plane wave and band (conversion and sums);
+// conversion 50e-6 per element. Measured (ZGEMMs -> residues, conversion) against the rule's choice:
+//   26,398 waves, 256 projectors: 96 bands 330 -> 308, 313 (ZGEMMs); 128 bands 434 -> 357, 326; 160 533 -> 410, 320
+//   34,809, 336: 64 bands 386 -> 372, 521 (ZGEMMs); 96 568 -> 431, 522
+//   89,137, 864: 32 bands 1,170 -> 1,306 (ZGEMMs); 64 2,260 -> 1,464, 3,010; 240 8,667 -> 2,595, 3,026
+//   9,898, 700: 64 bands 248 -> 211, 459 (ZGEMMs); 160 564 -> 255, 454; 89,137, 200: 96 bands 925 -> 888, 840 (ZGEMMs)
+//   89,137, 64, 480 bands: 1,511 -> 3,019; 34,809, 100, 300 bands: 674 -> 843 (ZGEMMs)
+//
+// MIXED_TC, where the other form is split TF32 and differs by ~1e-7: by the projector set alone, so that a
+// band's result does not depend on the other bands of its call. Sets of kResidueElements elements of X, where
+// residues are no more than 8 % slower at any number of bands (17.8 M elements: 263 -> 240 at 4 bands, 314 ->
+// 337 at 64, 449 -> 440 at 128, 1,033 -> 770 at 270) and the conversion no more than the split (13.7 M: 240 -> 280
+// at 64 bands; 6.8 M: 126 -> 131 at 4, 211 -> 253 at 128, 311 -> 296 at 160; 77 M: 892 -> 702 at 4, 2,961 -> 1,726
+// at 240, conversion 2,300 against 3,400).
+constexpr double kResidueCalls = 8, kResidueElements = 1.6e7;
 bool residues_pay(int precision, int m, int nanl, int nb) {
   // int32 sums, a grid dimension, 16-bit sums over the K splits
   if (nanl <= 0 || nanl > kCrtMaxProjectors || nb > 65535 || m > 15000000) return false;
   if (const char* v = getenv("CPW_B200_NL_CRT")) return atoi(v) != 0;
-  const double flops = 16.0 * m * nanl * nb;
-  return precision == 2 ? nb >= 128 && flops >= 1.5e10 : nb >= 64 && flops >= 1e10;
+  const double elements = (double)m * nanl, waves = (double)m * nb;
+  if (precision == 2) return elements >= kResidueElements;
+  const double zgemm = 16.0 * elements * nb / 33e6, residues = 75 + 15e-6 * elements + 55e-6 * waves;
+  return kResidueCalls * (zgemm - residues) >= 50e-6 * elements;
 }
 static bool crt_pays(const cpw_b200_ctx* c, int nb) {
   // a MIXED_TC solve keeps split TF32 for all its blocks (ditsp.cu)

@@ -57,3 +57,52 @@ def test_a_mixed_solve_keeps_one_form(cuda):
         pass                                # the small matrix is another operator's: no convergence is asked for
     assert _taken(alone, ctx.form_counts()) == {"split_tf32"}
     ctx.close()
+
+
+def _forms(cuda, ctx, m, nbs):
+    import torch
+    out = {}
+    for nb in nbs:
+        psi = torch.randn((nb, m), dtype=torch.complex128, device=cuda).t()
+        before = ctx.form_counts()
+        ctx.hk_psi(psi, torch.zeros_like(psi))
+        (out[nb],) = _taken(before, ctx.form_counts())
+    ctx.synchronize()
+    ctx.close()
+    return out
+
+
+def test_mixed_tc_form_follows_the_projector_set(cuda):
+    """16 M elements of X: below, split TF32 for any number of bands; above, residues."""
+    d = configs.kpoint_inputs(configs.si8_cubic_kbatch(nk=1), 0)
+    m = d["mtxd"]
+    na = int(1.6e7 / m) + 1
+    assert set(_forms(cuda, _context(d, H.MIXED_TC, na), m, (1, 60, 140)).values()) == {"residues"}
+    assert set(_forms(cuda, _context(d, H.MIXED_TC, na - 1), m, (1, 60, 140)).values()) == {"split_tf32"}
+
+
+@pytest.mark.parametrize("na,nb,form", [(700, 60, "zgemm"), (700, 200, "residues"), (32, 400, "zgemm"),
+                                        (64, 600, "zgemm")])
+def test_fp64_form_counts_the_conversion(cuda, na, nb, form):
+    """The rule's sides, among them many bands on few projectors, which ZGEMMs do faster at any size."""
+    d = configs.kpoint_inputs(configs.si8_cubic_kbatch(nk=1), 0)
+    assert _forms(cuda, _context(d, H.FP64, na), d["mtxd"], (nb,)) == {nb: form}
+
+
+def test_drop_in_with_both_forms_in_one_call(cuda):
+    """831 plane waves, 4,200 projectors: six chunks whose four inner ones (96 bands) take residues and whose half-size
+    ends take ZGEMMs."""
+    from oracle import hk_psi as O
+    d = configs.kpoint_inputs(configs.si2_fcc(), 1)
+    m, na, nb = d["mtxd"], 4200, 480
+    x, xnl = _projectors(m, na)
+    x = np.asfortranarray(x)
+    psi = configs.random_psi(m, nb, 5)
+    hpsi = np.zeros((m, nb), dtype=np.complex128, order="F")
+    before = H.form_counts()
+    H.hk_psi_c16(m, nb, psi, hpsi, False, d["ng"], np.asfortranarray(d["kgv"]), d["ekpg"], d["isort"], d["vscr"],
+                 d["kmscr"], x, xnl, na, m, nb, na, d["ng"], d["vscr"].size)
+    after = H.form_counts()
+    assert {k: after[k] - before[k] for k in _taken(before, after)} == {"residues": 4, "zgemm": 2}
+    ref = O.hk_psi_c16(m, nb, psi, d["ekpg"], d["isort"], d["vscr"], d["kmscr"], d["kgv"], x, xnl)
+    assert np.abs(hpsi - ref).max() < 1e-12 * np.abs(ref).max()
