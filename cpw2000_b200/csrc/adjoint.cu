@@ -226,16 +226,17 @@ __global__ void k_to_complex(long long n, const double* __restrict__ g, Z* __res
     z[t] = make_cuDoubleComplex(g[t], 0.0);
 }
 
-// c[a][j] = sum_i Im(conj(X_ia) Y_ia) G_ij, one CTA per projector
+// c[slice][a][j] = sum_i Im(conj(X_ia) Y_ia) G_ij over the slice's plane waves, one CTA per projector and slice
 __global__ void __launch_bounds__(256) k_nl_contract(int m, const int* __restrict__ kgvb, const Z* __restrict__ X,
-                                                     const Z* __restrict__ Y, double* __restrict__ c) {
-  const int a = blockIdx.x;
+                                                     const Z* __restrict__ Y, double* __restrict__ c, int nanl) {
+  const int a = blockIdx.x, rows = (m + gridDim.y - 1) / gridDim.y;
+  const int i1 = min(m, ((int)blockIdx.y + 1) * rows);
   __shared__ double sh[32];
   double s[3] = {0, 0, 0};
   const Z* x = X + (size_t)a * m;
   const Z* y = Y + (size_t)a * m;
 #pragma unroll 2
-  for (int i = threadIdx.x; i < m; i += 256) {
+  for (int i = blockIdx.y * rows + threadIdx.x; i < i1; i += 256) {
     const Z p = x[i], q = y[i];
     const double w = p.x * q.y - p.y * q.x;
     s[0] += w * kgvb[3 * i];
@@ -244,7 +245,7 @@ __global__ void __launch_bounds__(256) k_nl_contract(int m, const int* __restric
   }
   for (int j = 0; j < 3; ++j) {
     const double t = block_sum3(s[j], sh);
-    if (threadIdx.x == 0) c[3 * a + j] = t;
+    if (threadIdx.x == 0) c[3 * ((size_t)blockIdx.y * nanl + a) + j] = t;
   }
 }
 
@@ -467,11 +468,18 @@ int nl_grad_device(cpw_b200_ctx* c, int nb, const void* psi, long long ldpsi, co
   for (int a = 0; a < na; ++a)
     if (proj_atom[a] < 0 || proj_atom[a] >= natom) return fail(kBadArg, "projector gradient: proj_atom out of range");
   // With Y = psi diag(f) P^H the sum over bands goes first: sum_n f_n Im(conj(P_an) Q_jan) =
-  // Im sum_i conj(X_ia) G_ij Y_ia, one product of the size of P's in place of the three X^H (G_j psi)
-  // (26,529 plane waves, 256 projectors, 128 bands: 694 us with the scaled copies of psi -> 221 for Y and 82 for the contraction)
-  const size_t zP = sizeof(Z) * (size_t)na * nb, zY = sizeof(Z) * (size_t)m * na;
+  // Im sum_i conj(X_ia) G_ij Y_ia, one product of the size of P's in place of the three X^H (G_j psi).
+  // The work space is kept, so Y is made in blocks of projectors of at most 512 MB (64 projectors at least, a tile
+  // of the product). us for 4 and 128 bands: 26,398 plane waves, 256 projectors, one block of 108 MB, 214 and
+  // 535; 89,137, 864, blocks of 64 MB, 256 MB, 512 MB and whole (1.2 GB): 1,738, 1,667, 1,525, 1,474 and 5,411,
+  // 5,379, 5,139, 5,100. The contraction's plane waves are split into slices, which fill the SMs for few projectors too.
+  const size_t colY = sizeof(Z) * (size_t)m;
+  const int most = std::max(64, (int)std::min<size_t>((size_t)na, (size_t)(512 << 20) / colY / 32 * 32));
+  const int blocks = (na + most - 1) / most, per = std::min(na, ((na + blocks - 1) / blocks + 31) / 32 * 32);
+  const int slices = std::max(1, std::min(16, (592 + per - 1) / per));       // about four CTAs per SM in the contraction
+  const size_t zP = sizeof(Z) * (size_t)na * nb, zY = colY * per;
   int s;
-  if ((s = c->adj.ensure(zY + 2 * zP + sizeof(double) * (3 * (size_t)na + nb)))) return s;
+  if ((s = c->adj.ensure(zY + 2 * zP + sizeof(double) * (3 * (size_t)na * slices + nb)))) return s;
   char* base = (char*)c->adj.p;
   Z* Y = (Z*)base;
   Z* P = (Z*)(base + zY);
@@ -487,16 +495,25 @@ int nl_grad_device(cpw_b200_ctx* c, int nb, const void* psi, long long ldpsi, co
   if (bs != CUBLAS_STATUS_SUCCESS) return fail(kCublas, "projector gradient zgemm P");
   k_stress_m<<<(int)std::max(1LL, std::min(1184LL, ((long long)na * nb + 255) / 256)), 256, 0, st>>>(
       na, nb, P, docc, nullptr, M);
-  bs = cublasZgemm(c->blas, CUBLAS_OP_N, CUBLAS_OP_N, m, na, nb, &one, (const Z*)psi, (int)ldpsi, M, nb, &zero, Y, m);
-  if (bs != CUBLAS_STATUS_SUCCESS) return fail(kCublas, "projector gradient zgemm Y");
-  k_nl_contract<<<na, 256, 0, st>>>(m, (const int*)c->kgvb.p, (const Z*)c->anl.p, Y, dc);
-  std::vector<double> ch(3 * (size_t)na);
-  e = cudaMemcpyAsync(ch.data(), dc, sizeof(double) * 3 * na, cudaMemcpyDeviceToHost, st);
+  for (int a0 = 0; a0 < na; a0 += per) {
+    const int n = std::min(per, na - a0);
+    bs = cublasZgemm(c->blas, CUBLAS_OP_N, CUBLAS_OP_N, m, n, nb, &one, (const Z*)psi, (int)ldpsi, M + (size_t)a0 * nb,
+                     nb, &zero, Y, m);
+    if (bs != CUBLAS_STATUS_SUCCESS) return fail(kCublas, "projector gradient zgemm Y");
+    k_nl_contract<<<dim3(n, slices), 256, 0, st>>>(m, (const int*)c->kgvb.p, (const Z*)c->anl.p + (size_t)a0 * m, Y,
+                                                   dc + 3 * (size_t)a0, na);
+  }
+  std::vector<double> ch(3 * (size_t)na * slices);
+  e = cudaMemcpyAsync(ch.data(), dc, sizeof(double) * ch.size(), cudaMemcpyDeviceToHost, st);
   if (e != cudaSuccess) return cuda_fail(e, "projector gradient copy");
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return cuda_fail(e, "projector gradient");
   const double fpi = 12.566370614359172953850573533118011537;
   for (int a = 0; a < na; ++a)
-    for (int j = 0; j < 3; ++j) dedtau[3 * proj_atom[a] + j] += -fpi * c->xnl_h[a] * ch[3 * (size_t)a + j];
+    for (int j = 0; j < 3; ++j) {
+      double t = 0.0;
+      for (int k = 0; k < slices; ++k) t += ch[3 * ((size_t)k * na + a) + j];
+      dedtau[3 * proj_atom[a] + j] += -fpi * c->xnl_h[a] * t;
+    }
   return kOk;
 }
 

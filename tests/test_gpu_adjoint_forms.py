@@ -113,3 +113,33 @@ def test_structure_gradient(cuda, box, counts):
         ref[a] = 2 * np.pi * np.array([(w * m[0]).sum(), (w * m[1][:, None]).sum(), (w * m[2][:, None, None]).sum()])
     assert np.abs(out - ref).max() < 1e-12 * np.abs(ref).max()
     ctx.close()
+
+
+@pytest.mark.parametrize("na,nb", [(1, 3), (64, 1), (65, 4), (900, 2), (7400, 1)])
+def test_projector_gradient_over_slices(cuda, na, nb):
+    """One projector (16 slices of plane waves), more projectors than CTAs, and two blocks of projectors (7,400 on
+    4,613 plane waves are 546 MB), against numpy: FP64 sums, 1e-12 of the largest product's scale."""
+    import torch
+    from cpw2000_b200 import configs
+    d = configs.kpoint_inputs(configs.si8_cubic_kbatch(nk=1), 0)
+    m, natom = d["mtxd"], 3
+    rng = np.random.default_rng(na)
+    x = np.resize(rng.standard_normal((1 << 20) - 3), 2 * m * na).view(np.complex128).reshape(na, m).T
+    xnl, occ = rng.choice((-1.0, 1.0), na), np.linspace(2.0, 0.5, nb)
+    atom = rng.integers(0, natom, na).astype(np.int32)
+    psi = rng.standard_normal((m, nb)) + 1j * rng.standard_normal((m, nb))
+    ctx = H.Context(0)
+    ctx.set_kpoint(m, d["isort"], d["kgv"], d["ekpg"], d["kmscr"])
+    ctx.set_potential(d["vscr"])
+    ctx.set_projectors(x, xnl)
+    p, out = _dev(cuda, psi), np.zeros((natom, 3))
+    _lib.check(_lib.lib().cpw_b200_nl_grad_device(ctx.handle, nb, C.c_void_p(p.data_ptr()), m, _lib.dptr(occ),
+                                                  _lib.iptr(atom), natom, _lib.dptr(out), None))
+    g = d["kgv"][:, d["isort"] - 1].astype(float)
+    pr = x.conj().T @ psi
+    ref = np.zeros((natom, 3))
+    for j in range(3):
+        q = x.conj().T @ (g[j][:, None] * psi)
+        np.add.at(ref[:, j], atom, -4 * np.pi * xnl * ((pr.conj() * q).imag @ occ))
+    assert np.abs(out - ref).max() < 1e-12 * np.abs(pr).max() ** 2 * np.abs(g).max() * na
+    ctx.close()
