@@ -331,7 +331,8 @@ int density_device(cpw_b200_ctx* c, int nb, const void* psi, long long ldpsi, co
   // the y tile of a context with FP32 transforms was fitted for their element size
   int smax = 0;
   cudaDeviceGetAttribute(&smax, cudaDevAttrMaxSharedMemoryPerBlockOptin, c->device);
-  if (p.tcol > 32 && smem_planes<double>(p) > (size_t)smax) p.tcol = 32;
+  if (!plane_tile(sizeof(C2<double>), p, (size_t)smax))
+    return fail(kUnsupported, "density: plane does not fit in shared memory");
   cudaError_t e = cudaMemsetAsync(rho, 0, sizeof(double) * (size_t)p.plane * p.n3, st);
   if (e != cudaSuccess) return cuda_fail(e, "density memset");
   if (nb == 0 || c->mtxd == 0) return kOk;

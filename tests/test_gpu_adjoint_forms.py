@@ -40,9 +40,10 @@ def test_density(cuda, n3, inside):
     _density(cuda, (10, 9, n3), (2, 2, _kd3(n3, inside)), H.FP64)
 
 
-def test_density_wide_plane_of_a_mixed_context(cuda):
-    # a y tile of 40 columns fits the shared memory in FP32, one of 32 in FP64
-    _density(cuda, (40, 256, 16), (2, 54, 2), H.MIXED)
+@pytest.mark.parametrize("box,kd", [((40, 256, 16), (2, 54, 2)), ((144, 144, 16), (2, 34, 2))])
+def test_density_wide_plane_of_a_mixed_context(cuda, box, kd):
+    # a y tile of 40 columns fits the shared memory in FP32, one of 32 in FP64; one of 32 in FP32, one of 16 in FP64
+    _density(cuda, box, kd, H.MIXED)
 
 
 def _density(cuda, box, kd, prec):
