@@ -105,8 +105,9 @@ int d2h_cols(double* dst, long long ldd, const void* src, long long lds, long lo
 // band chunks: every chunk's copy to the device is issued first on its own stream (the caller
 // checks its other inputs on the host meanwhile), chunk k is computed once its copy landed, and
 // its copy back runs on a third stream while chunk k+1 is computed (with page-locked host
-// arrays the three overlap; pageable arrays degrade to staged copies). Results are the same
-// as one pass: every band's H|psi> depends on that band only.
+// arrays the three overlap; pageable arrays degrade to staged copies). Every band's H|psi>
+// depends on that band only; its projector products take the form of its chunk's size (residues
+// or ZGEMMs of the same accuracy, both within one call where the end chunks are too small).
 struct DropinPipe {
   int m = 0, nb = 0, chunk = 0, nchunk = 0;
   long long ldh = 0;

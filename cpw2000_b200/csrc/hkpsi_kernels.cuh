@@ -250,8 +250,8 @@ k_z_vloc(LocalPlan p, const T* __restrict__ vr, const C2<T>* __restrict__ twz, C
         constexpr int RR = decltype(rc_)::value;
         C2<T> v[RR];
         T vz[RR];
+        const int vc = slab_column(p, c0 + cl);
 #pragma unroll
-        const long long vc = slab_column(p, c0 + cl);
         for (int a = 0; a < RR; ++a) vz[a] = vr[(size_t)(k1 + r1 * a) * p.plane + vc];
 #pragma unroll
         for (int a = 0; a < RR; ++a) v[a] = Cs[(size_t)(r2 * k1 + a) * cb + cl];

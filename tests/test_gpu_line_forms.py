@@ -93,3 +93,8 @@ def test_band_groups_and_chunks_do_not_change_a_bit(cuda):
     ctx.hk_psi(x, part)
     assert torch.equal(whole, part)
     ctx.close()
+
+
+def test_line_that_fits_no_staging(cuda):
+    # 255 kept planes of 256: two staging buffers exceed the shared memory of a CTA in FP64 (the plain form of B)
+    _check(cuda, (10, 9, 256), (2, 2, 127), 3, H.FP64, 1)
