@@ -18,11 +18,12 @@ constexpr int kThreadsCols = 256;
 // CTAs per SM asked of the register allocator for kernels A and C (fwd): the passes wait on shared memory
 // and on the plane's loads, so small planes want as many CTAs as their shared memory lets in. us per launch
 // with this bound, before -> after:
-//   40 x 40 (320 threads; 2,560 bands FP32, 160 FP64): C FP32 three -> five 541 -> 404 (six the same), A FP32
-//   four -> six 361 -> 326; C FP64 two -> three 60 -> 52 (four 52 with the read-ahead gather that takes three
-//   to 46), A FP64 three -> four 36 -> 35.
-//   96 x 96 FP32 (160 bands): C with 384 threads in three CTAs 164, 256 in three 179, 256 in four 210;
-//   A in three 139, in four 160 (spills).
+//   Up to 64 points (10 to 40 KB a plane). 40 x 40 (320 threads; 2,560 bands FP32, 160 FP64): C FP32 three -> five 541
+//   -> 404 (six the same), A FP32 four -> six 361 -> 326; C FP64 two -> three 60 -> 52 (four 52 with the read-ahead
+//   gather that takes three to 46), A FP64 three -> four 36 -> 35. 32 x 32 x 96 (256 threads, 1,000 bands), no
+//   bound -> this one: A FP32 139 -> 128, C FP32 157 and both FP64 205 and 236 unchanged.
+//   FP32 planes of 65 to 127 points (64 KB at 96, three to an SM). 96 x 96 (160 bands): C with 384 threads in three
+//   CTAs 164, 256 in three 179, 256 in four 210; A in three 139, in four 160 (spills).
 //   FP64 planes of 128 points or more take over 200 KB of shared memory, one CTA per SM whatever the
 //   registers: no cap. The others: two CTAs of 384 threads in 80 registers.
 // The run-time form (n1 = 0) would take the registers of its largest radix, one CTA of 256 threads per SM in
@@ -30,9 +31,9 @@ constexpr int kThreadsCols = 256;
 // memory lets them in (many: 64 x 50, 91 bands, C 96 -> 83, A 81 -> 72; 48 bands of 48 x 48 42 -> 38 for
 // both, 72 x 72 76 -> 73; 80 x 80, which would hold four, 98 -> 111).
 template <typename T> constexpr int plane_min_blocks(int nt, int n1, bool fwd, bool many) {
-  if (n1 == 40) return sizeof(T) == 8 ? (fwd ? 3 : 4) : fwd ? 5 : 6;
-  if (n1 == 96 && sizeof(T) == 4) return 3;
   if (n1 == 0) return sizeof(T) == 8 ? 2 : many ? 5 : 3;
+  if (n1 <= 64) return sizeof(T) == 8 ? (fwd ? 3 : 4) : fwd ? 5 : 6;
+  if (n1 < 128 && sizeof(T) == 4) return 3;
   return sizeof(T) == 8 && n1 >= 128 ? 1 : nt >= 320 ? 2 : 1;
 }
 constexpr size_t kManyPlaneBytes = 44 * 1024;   // five CTAs to an SM
