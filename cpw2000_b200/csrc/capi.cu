@@ -510,6 +510,7 @@ int cpw_b200_zgemm_i8_tri(cpw_b200_ctx* c, int transa, int m, int n, int k, cons
                           const void* b, long long ldb, double alpha, int accumulate, void* cm, long long ldc,
                           int slices, int tri, void* stream) {
   if (int s = check_ctx(c)) return s;
+  const SpareMemory spare(c);
   if (tri < 0 || tri > 2) return fail(kBadArg, "zgemm_i8: tri must be 0, 1 or 2");
   if (transa != 'N' && transa != 'C') return fail(kBadArg, "zgemm_i8: transa must be 'N' or 'C'");
   if (m < 0 || n < 0 || k < 0) return fail(kBadArg, "zgemm_i8: negative dimension");
@@ -555,24 +556,28 @@ int cpw_b200_timing_end(cpw_b200_ctx* c, double* ms, long long* launches, int ns
 int cpw_b200_set_kpoint(cpw_b200_ctx* c, int mtxd, const int* isort, const int* kgv, int ng, const double* ekpg,
                         const int* kmscr) {
   if (int s = check_ctx(c)) return s;
+  const SpareMemory spare(c);
   cudaSetDevice(c->device);
   return ctx_set_basis(c, mtxd, isort, kgv, ng, ekpg, kmscr);
 }
 
 int cpw_b200_set_potential(cpw_b200_ctx* c, const double* vscr, long long mxdscr) {
   if (int s = check_ctx(c)) return s;
+  const SpareMemory spare(c);
   cudaSetDevice(c->device);
   return ctx_set_potential(c, vscr, mxdscr);
 }
 
 int cpw_b200_set_projectors(cpw_b200_ctx* c, int nanl, const double* anlga, int mxddim, const double* xnlkb) {
   if (int s = check_ctx(c)) return s;
+  const SpareMemory spare(c);
   cudaSetDevice(c->device);
   return ctx_set_projectors(c, nanl, anlga, mxddim, xnlkb, false);
 }
 
 int cpw_b200_set_projectors_device(cpw_b200_ctx* c, int nanl, const void* anlga, int ld, const void* xnlkb) {
   if (int s = check_ctx(c)) return s;
+  const SpareMemory spare(c);
   cudaSetDevice(c->device);
   return ctx_set_projectors(c, nanl, (const double*)anlga, ld, (const double*)xnlkb, true);
 }
@@ -582,6 +587,7 @@ int cpw_b200_proj_nl_kb_device(cpw_b200_ctx* c, const double* rkpt, int ntype, c
                                const double* vkb, int mxdlqp, const int* nkb, int nanl, double* xnlkb,
                                void* anlga, long long ldanl) {
   if (int s = check_ctx(c)) return s;
+  const SpareMemory spare(c);
   cudaSetDevice(c->device);
   return ctx_proj_nl_kb(c, rkpt, ntype, natom, rat, mxdatm, adot, nqnl, delqnl, vkb, mxdlqp, nkb, nanl, xnlkb, anlga,
                         ldanl);
@@ -593,6 +599,7 @@ int cpw_b200_proj_nl_kb_der_device(cpw_b200_ctx* c, int nder, const double* rkpt
                                    double* xnlkb, void* anlga, long long ld, long long mxdanl, void* danlgadrk,
                                    void* d2anlgadrk2) {
   if (int s = check_ctx(c)) return s;
+  const SpareMemory spare(c);
   cudaSetDevice(c->device);
   return ctx_proj_nl_kb_der(c, nder, rkpt, ntype, natom, rat, mxdatm, adot, nqnl, delqnl, vkb, mxdlqp, nkb, nanl,
                             xnlkb, anlga, ld, mxdanl, danlgadrk, d2anlgadrk2);
@@ -605,6 +612,7 @@ int cpw_b200_hamilt_kb_device(cpw_b200_ctx* c, int mtxd, const double* hdiag, co
                               const int* nkb, int ntype, const double* adot, void* hamk, long long ldh, int mxdtyp,
                               int mxdgve, int mxdnst, int mxdcub, int mxdlqp, int mxddim) {
   if (int s = check_ctx(c)) return s;
+  const SpareMemory spare(c);
   cudaSetDevice(c->device);
   return hamilt_kb_device(c, mtxd, hdiag, isort, qmod, ng, kgv, phase, conj, inds, kmax, indv, ek, sfact, veff, nqnl,
                           delqnl, vkb, nkb, ntype, adot, hamk, ldh, mxdtyp, mxdgve, mxdnst, mxdcub, mxdlqp, mxddim);
@@ -614,6 +622,7 @@ int cpw_b200_pot_local(cpw_b200_ctx* c, double* vscr, double* vmax, double* vmin
                        int* kmscr, int idshift, int ng, const int* kgv, const double* phase, const double* conj, int ns,
                        const int* inds, int mxdscr, int mxdgve, int mxdnst, int install) {
   if (int s = check_ctx(c)) return s;
+  const SpareMemory spare(c);
   // the checks of pot_local.f90:104-120 and the bounds it assumes
   if (ng < 0 || ng > mxdgve) return fail(kBadArg, "pot_local: ng out of range of mxdgve");
   if (ns < 0 || ns > mxdnst) return fail(kBadArg, "pot_local: ns out of range of mxdnst");
@@ -642,6 +651,7 @@ int cpw_b200_pot_local(cpw_b200_ctx* c, double* vscr, double* vmax, double* vmin
 int cpw_b200_hk_psi_kin_device(cpw_b200_ctx* c, int neig, const void* psi, long long ldpsi, void* hpsi, long long ldh,
                                int ladd, int nspin, void* stream) {
   if (int s = check_ctx(c)) return s;
+  const SpareMemory spare(c);
   cudaSetDevice(c->device);
   cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
   return ctx_hkpsi_kin_device(c, neig, psi, ldpsi, hpsi, ldh, ladd != 0, nspin, st);
@@ -650,6 +660,7 @@ int cpw_b200_hk_psi_kin_device(cpw_b200_ctx* c, int neig, const void* psi, long 
 int cpw_b200_hk_psi_loc_c16_device(cpw_b200_ctx* c, int neig, const void* psi, long long ldpsi, void* hpsi,
                                    long long ldh, int ladd, int nspin, void* stream) {
   if (int s = check_ctx(c)) return s;
+  const SpareMemory spare(c);
   cudaSetDevice(c->device);
   cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
   return ctx_hkpsi_loc_general(c, neig, psi, ldpsi, hpsi, ldh, ladd != 0, nspin, st);
@@ -657,12 +668,14 @@ int cpw_b200_hk_psi_loc_c16_device(cpw_b200_ctx* c, int neig, const void* psi, l
 
 int cpw_b200_set_potential_spin(cpw_b200_ctx* c, const double* vscr_sp, long long mxdscr, int nsp) {
   if (int s = check_ctx(c)) return s;
+  const SpareMemory spare(c);
   cudaSetDevice(c->device);
   return ctx_set_potential_spin(c, vscr_sp, mxdscr, nsp);
 }
 
 int cpw_b200_set_projectors_spin(cpw_b200_ctx* c, int nanlsp, const double* anlsp, long long ld, const double* xnlkbsp) {
   if (int s = check_ctx(c)) return s;
+  const SpareMemory spare(c);
   cudaSetDevice(c->device);
   return ctx_set_projectors_spin(c, nanlsp, anlsp, ld, xnlkbsp);
 }
@@ -670,6 +683,7 @@ int cpw_b200_set_projectors_spin(cpw_b200_ctx* c, int nanlsp, const double* anls
 int cpw_b200_hk_psi_spin_device(cpw_b200_ctx* c, int neig, const void* psi_sp, long long ldpsi, void* hpsi_sp,
                                 long long ldh, void* stream) {
   if (int s = check_ctx(c)) return s;
+  const SpareMemory spare(c);
   cudaSetDevice(c->device);
   cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
   return ctx_hkpsi_spin_device(c, neig, psi_sp, ldpsi, hpsi_sp, ldh, st);
@@ -678,6 +692,7 @@ int cpw_b200_hk_psi_spin_device(cpw_b200_ctx* c, int neig, const void* psi_sp, l
 int cpw_b200_hk_psi_device(cpw_b200_ctx* c, int neig, const void* psi, long long ldpsi, void* hpsi, long long ldh,
                            void* stream) {
   if (int s = check_ctx(c)) return s;
+  const SpareMemory spare(c);
   cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
   return ctx_hkpsi_device(c, neig, psi, ldpsi, hpsi, ldh, st, true, true);
 }
@@ -685,6 +700,7 @@ int cpw_b200_hk_psi_device(cpw_b200_ctx* c, int neig, const void* psi, long long
 int cpw_b200_hk_psi_loc_device(cpw_b200_ctx* c, int neig, const void* psi, long long ldpsi, void* hpsi,
                                long long ldh, void* stream) {
   if (int s = check_ctx(c)) return s;
+  const SpareMemory spare(c);
   cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
   return ctx_hkpsi_device(c, neig, psi, ldpsi, hpsi, ldh, st, false, false);
 }
@@ -714,6 +730,7 @@ int cpw_b200_hk_psi_c16(const int* mtxd, const int* neig, const double* psi, dou
   }
   cpw_b200_ctx* c;
   if (int s = default_ctx(&c)) return s;
+  const SpareMemory spare(c);
   cudaSetDevice(c->device);
   const int m = *mtxd, nb = *neig;
   int s;
@@ -876,6 +893,7 @@ int cpw_b200_ditsp_device(cpw_b200_ctx* c, int ipr, int* ifail, int icmax, int i
                           int mxdsml, const double* hdiag, int mxdbnd, long long* ihkpsum, void* stream,
                           double* itlog, int itlog_rows) {
   if (int s = check_ctx(c)) return s;
+  const SpareMemory spare(c);
   cudaSetDevice(c->device);
   cudaStream_t st = stream ? (cudaStream_t)stream : c->stream;
   long long ih = 0;
@@ -903,6 +921,7 @@ int cpw_b200_ditsp_c16(const int* ipr, int* ifail, const int* icmax, const int* 
   if (*ng > *mxdgve) return fail(kBadArg, "ditsp_c16: ng is greater than mxdgve");
   cpw_b200_ctx* c;
   if (int s = default_ctx(&c)) return s;
+  const SpareMemory spare(c);
   cudaSetDevice(c->device);
   const int m = *mtxd, nb = *mxdbnd;
   int s;
@@ -944,6 +963,7 @@ void ditsp_c16_(const int* ipr, int* ifail, const int* icmax, const int* iguess,
 int cpw_b200_density_device(cpw_b200_ctx* c, int neig, const void* psi, long long ldpsi, const double* occ,
                             void* rho, void* stream) {
   if (int s = check_ctx(c)) return s;
+  const SpareMemory spare(c);
   cudaSetDevice(c->device);
   return density_device(c, neig, psi, ldpsi, occ, rho, stream ? (cudaStream_t)stream : c->stream);
 }
@@ -951,6 +971,7 @@ int cpw_b200_density_device(cpw_b200_ctx* c, int neig, const void* psi, long lon
 int cpw_b200_structure_grad_device(cpw_b200_ctx* c, const void* g, int natom, const int* atom_type, const double* tau,
                                    int ntype, const void* vgt, double* dedtau, void* stream) {
   if (int s = check_ctx(c)) return s;
+  const SpareMemory spare(c);
   cudaSetDevice(c->device);
   return structure_grad_device(c, g, natom, atom_type, tau, ntype, vgt, dedtau,
                                stream ? (cudaStream_t)stream : c->stream);
@@ -959,6 +980,7 @@ int cpw_b200_structure_grad_device(cpw_b200_ctx* c, const void* g, int natom, co
 int cpw_b200_nl_grad_device(cpw_b200_ctx* c, int neig, const void* psi, long long ldpsi, const double* occ,
                             const int* proj_atom, int natom, double* dedtau, void* stream) {
   if (int s = check_ctx(c)) return s;
+  const SpareMemory spare(c);
   cudaSetDevice(c->device);
   return nl_grad_device(c, neig, psi, ldpsi, occ, proj_atom, natom, dedtau, stream ? (cudaStream_t)stream : c->stream);
 }
@@ -966,6 +988,7 @@ int cpw_b200_nl_grad_device(cpw_b200_ctx* c, int neig, const void* psi, long lon
 int cpw_b200_stress_inputs_device(cpw_b200_ctx* c, int neig, const void* psi, long long ldpsi, const double* occ,
                                   double* w, void* y, void* stream) {
   if (int s = check_ctx(c)) return s;
+  const SpareMemory spare(c);
   cudaSetDevice(c->device);
   return stress_inputs_device(c, neig, psi, ldpsi, occ, w, y, stream ? (cudaStream_t)stream : c->stream);
 }
@@ -980,6 +1003,7 @@ int cpw_b200_hk_psi_nl_c16(const int* mtxd, const int* neig, const double* psi, 
   if (m == 0 || nb == 0) return kOk;
   cpw_b200_ctx* c;
   if (int s = default_ctx(&c)) return s;
+  const SpareMemory spare(c);
   cudaSetDevice(c->device);
   DevBuf x, xd, p, h, v;
   int s;

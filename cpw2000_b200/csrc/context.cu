@@ -40,6 +40,21 @@ StageTimer::~StageTimer() {
   for (cudaEvent_t e : pool) cudaEventDestroy(e);
 }
 
+static thread_local cpw_b200_ctx* t_spare = nullptr;
+SpareMemory::SpareMemory(cpw_b200_ctx* c) : before(t_spare) { t_spare = c; }
+SpareMemory::~SpareMemory() { t_spare = before; }
+
+// Not what a graph may still read. cudaFree waits for the kernels that use the buffers.
+static bool take_back_residues() {
+  cpw_b200_ctx* c = t_spare;
+  if (!c || c->crt_making || !c->crt.captured.empty() || (!c->crt.buf.p && !c->crts.buf.p)) return false;
+  c->crt.buf.release();
+  c->crts.buf.release();
+  c->crt.L = 0;
+  c->crt_off = true;            // until the projectors change
+  return true;
+}
+
 int DevBuf::ensure(size_t need) {
   if (need <= bytes && p) return kOk;
   // a buffer that grows takes 1.5x (at least) of its old size, rounded to 2 MiB: buffers sized by
@@ -50,6 +65,10 @@ int DevBuf::ensure(size_t need) {
   release();
   if (need == 0) return kOk;
   cudaError_t e = cudaMalloc(&p, need);
+  if (e == cudaErrorMemoryAllocation && take_back_residues()) {
+    cudaGetLastError();
+    e = cudaMalloc(&p, need);
+  }
   if (e != cudaSuccess) {
     p = nullptr;
     bytes = 0;
@@ -352,6 +371,11 @@ static bool crt_ready(cpw_b200_ctx* c, int nb, cudaStream_t st) {
   const int L = residue_moduli(c);
   const bool have = c->crt.L == L && c->crt.m == c->mtxd && c->crt.na == c->nanl;
   if (!have && !free_run) return false;
+  struct Making {
+    cpw_b200_ctx* c;
+    ~Making() { c->crt_making = false; }
+  } making{c};
+  c->crt_making = true;
   if ((!have && crt_prepare(c->crt, c->mtxd, c->nanl, L, c->anl.p, c->anld.p, st)) ||
       crt_reserve(c->crts, c->crt, nb, free_run) || (free_run ? tc_error_flag(c->tcs) != kOk : !c->tcs.err.p)) {
     if (free_run) {

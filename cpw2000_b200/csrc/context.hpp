@@ -55,6 +55,15 @@ struct DevBuf {
   ~DevBuf() { release(); }
 };
 
+// While it lives, an allocation of this thread that fails first takes back the residue planes of context c, which
+// all calls can do without (their products then take the other form), and is tried once more.
+struct SpareMemory {
+  explicit SpareMemory(cpw_b200_ctx* c);
+  ~SpareMemory();
+  SpareMemory(const SpareMemory&) = delete;
+  cpw_b200_ctx* before;
+};
+
 int ditsp_device(cpw_b200_ctx* c, int ipr, int* ifail, int icmax, int iguess, double epspsi, int* neig_io, int mtxds,
                  void* psi, long long ldp, void* hpsi, const double* hamsm, int mxdsml, const double* hdiag,
                  int mxdbnd, double* ei, long long* ihkpsum, cudaStream_t st, double* itlog = nullptr,
@@ -200,6 +209,7 @@ struct cpw_b200_ctx {
   cpwb::CrtOperands crt;
   cpwb::CrtScratch crts;
   bool crt_off = false;
+  bool crt_making = false;      // being made: not to be taken back
   bool solving = false;         // inside ditsp_device
   long long tc_k1p = 0, tc_k2p = 0;     // K blocks (32 reals) of the projection and expansion operands
   bool tc_ready = false;

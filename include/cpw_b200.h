@@ -95,7 +95,9 @@ int cpw_b200_wait_selftest(cpw_b200_ctx* ctx, long long limit_ns, void* stream);
  * in any precision form; 0 restores the form's default (FP64 and MIXED:
  * residue GEMMs with 15 moduli for blocks large enough to pay for their
  * conversion, else cuBLAS FP64 ZGEMMs; MIXED_TC: 9 moduli or split-TF32
- * tensor-core GEMMs). 7 slices give
+ * tensor-core GEMMs). The residues of X and X D take 90 (MIXED_TC 54) bytes per
+ * element of X beside its own 32, and a call's scratch; they are given back when
+ * another allocation of the context fails. 7 slices give
  * FP64-level products (~2^-48 of the row maxima); 4 give ~2^-27, without the
  * bias of FP32 accumulation (the integer sums are exact). */
 int cpw_b200_set_projector_slices(cpw_b200_ctx* ctx, int slices);

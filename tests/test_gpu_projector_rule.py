@@ -106,3 +106,43 @@ def test_drop_in_with_both_forms_in_one_call(cuda):
     assert {k: after[k] - before[k] for k in _taken(before, after)} == {"residues": 4, "zgemm": 2}
     ref = O.hk_psi_c16(m, nb, psi, d["ekpg"], d["isort"], d["vscr"], d["kmscr"], d["kgv"], x, xnl)
     assert np.abs(hpsi - ref).max() < 1e-12 * np.abs(ref).max()
+
+
+def test_planes_make_room(cuda, monkeypatch):
+    """With the device nearly full, a call whose slab no longer fits takes the residue planes back and uses the other
+    form; so does one on new projectors whose planes do not fit; there is room again, and they come back."""
+    import torch
+    d = configs.kpoint_inputs(configs.si8_cubic_kbatch(nk=1), 0)
+    m, nb = d["mtxd"], 200
+    ctx = _context(d, H.FP64, 1500)         # planes 620 MB; a slab of 200 bands 108 MB
+    ctx.set_slab_budget(1 << 30)
+    psi = torch.randn((nb, m), dtype=torch.complex128, device=cuda).t()
+    few, full, again = torch.zeros_like(psi), torch.zeros_like(psi), torch.zeros_like(psi)
+    ctx.hk_psi(psi, few, neig=40)
+    before = ctx.form_counts()
+    monkeypatch.setenv("CPW_B200_NL_CRT", "1")
+    ctx.hk_psi(psi, few, neig=40)
+    monkeypatch.delenv("CPW_B200_NL_CRT")
+    assert _taken(before, ctx.form_counts()) == {"residues"}
+    ctx.synchronize()
+    torch.cuda.empty_cache()
+    fill = torch.empty(torch.cuda.mem_get_info()[0] - (32 << 20), dtype=torch.uint8, device=cuda)
+    before = ctx.form_counts()
+    ctx.hk_psi(psi, full)
+    ctx.synchronize()
+    assert _taken(before, ctx.form_counts()) == {"zgemm"}
+    ctx.set_projectors(*_projectors(m, 1500))
+    before = ctx.form_counts()
+    ctx.hk_psi(psi, again)
+    ctx.synchronize()
+    assert _taken(before, ctx.form_counts()) == {"zgemm"}
+    assert torch.equal(again, full)
+    del fill
+    torch.cuda.empty_cache()
+    ctx.set_projectors(*_projectors(m, 1500))
+    before = ctx.form_counts()
+    ctx.hk_psi(psi, again)
+    ctx.synchronize()
+    assert _taken(before, ctx.form_counts()) == {"residues"}
+    assert float((again - full).abs().max() / full.abs().max()) < 1e-12
+    ctx.close()
