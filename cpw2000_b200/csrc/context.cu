@@ -370,7 +370,8 @@ static bool crt_ready(cpw_b200_ctx* c, int nb, cudaStream_t st) {
   const bool free_run = cap == cudaStreamCaptureStatusNone;
   const int L = residue_moduli(c);
   const bool have = c->crt.L == L && c->crt.m == c->mtxd && c->crt.na == c->nanl;
-  if (!have && !free_run) return false;
+  // projectors that no eager call has converted: the conversion becomes part of the graph
+  if (!have && !free_run && c->crt.buf.bytes < crt_plane_bytes(c->mtxd, c->nanl, L)) return false;
   struct Making {
     cpw_b200_ctx* c;
     ~Making() { c->crt_making = false; }
@@ -390,6 +391,7 @@ static bool crt_ready(cpw_b200_ctx* c, int nb, cudaStream_t st) {
   const CrtOperands::Shape now{c->mtxd, c->nanl, L};
   auto& used = c->crt.captured;
   if (!free_run && std::find(used.begin(), used.end(), now) == used.end()) used.push_back(now);
+  c->crt_in_graph = !have && !free_run;
   return true;
 }
 
@@ -504,7 +506,9 @@ int ctx_hkpsi_device(cpw_b200_ctx* c, int nb, const void* psi, long long ldpsi, 
     cudaEvent_t t0 = c->timer.on ? c->timer.take() : nullptr, t1 = c->timer.on ? c->timer.take() : nullptr;
     cudaEvent_t t2 = c->timer.on ? c->timer.take() : nullptr;
     ++c->forms[kFormResidues];
-    if ((s = crt_nl_apply(c->crts, c->crt, nb, psi, ldpsi, hpsi, ldh, c->tcs, st, t0, t1, t2))) return s;
+    s = crt_nl_apply(c->crts, c->crt, nb, psi, ldpsi, hpsi, ldh, c->tcs, st, t0, t1, t2);
+    if (c->crt_in_graph) c->crt.L = 0;          // only a replay has the planes
+    if (s) return s;
     c->timer.mark(kStNlProj, t0, t1);
     c->timer.mark(kStNlExpand, t1, t2);
     return kOk;

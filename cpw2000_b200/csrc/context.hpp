@@ -135,6 +135,7 @@ struct CrtOperands {
 struct CrtScratch {
   DevBuf buf;
 };
+size_t crt_plane_bytes(int m, int na, int L);
 int crt_prepare(CrtOperands& o, int m, int na, int L, const void* anl, const void* anld, cudaStream_t st);
 int crt_reserve(CrtScratch& t, const CrtOperands& o, int nb, bool may_allocate);
 int crt_nl_apply(CrtScratch& t, const CrtOperands& o, int nb, const void* psi, long long ldpsi, void* hpsi,
@@ -210,6 +211,7 @@ struct cpw_b200_ctx {
   cpwb::CrtScratch crts;
   bool crt_off = false;
   bool crt_making = false;      // being made: not to be taken back
+  bool crt_in_graph = false;    // the call being captured converts the projectors itself
   bool solving = false;         // inside ditsp_device
   long long tc_k1p = 0, tc_k2p = 0;     // K blocks (32 reals) of the projection and expansion operands
   bool tc_ready = false;

@@ -734,6 +734,23 @@ int num_sms() {
 
 }  // namespace crt
 
+// One buffer: planes of X, planes of X D, row scales of both, partial norms (each cudaMalloc costs a few hundred
+// microseconds). Rows past the last one of a tile stay undefined: what they give is not read.
+struct CrtPlanes {
+  size_t b1, b2, bs, total;
+};
+static CrtPlanes planes_of(int m, int na, int L) {
+  using namespace crt;
+  CrtPlanes y{};
+  const size_t row = 3 * (size_t)L * kATile;
+  y.b1 = row * ((na + BM - 1) / BM) * ((m + KB - 1) / KB);
+  y.b2 = row * ((m + BM - 1) / BM) * ((na + KB - 1) / KB);
+  y.bs = align256(sizeof(int) * ((size_t)na + m));
+  y.total = y.b1 + y.b2 + y.bs + sizeof(Norm) * (size_t)((m + kNormChunk - 1) / kNormChunk) * na;
+  return y;
+}
+size_t crt_plane_bytes(int m, int na, int L) { return planes_of(m, na, L).total; }
+
 // Convert X (anl, m x na, ld m) and X D (anld) once per projector set, on st: a call on another stream is ordered
 // behind it as behind any earlier call, whose slab and scratch it shares.
 int crt_prepare(CrtOperands& o, int m, int na, int L, const void* anl, const void* anld, cudaStream_t st) {
@@ -744,17 +761,14 @@ int crt_prepare(CrtOperands& o, int m, int na, int L, const void* anl, const voi
   o.nkb2 = (na + KB - 1) / KB;
   o.tiles1 = (na + BM - 1) / BM;
   o.tiles2 = (m + BM - 1) / BM;
-  // one buffer: planes of X, planes of X D, row scales of both, partial norms (each cudaMalloc costs a
-  // few hundred microseconds). Rows past the last one of a tile stay undefined: what they give is not read.
   const int nchunk = (m + kNormChunk - 1) / kNormChunk;
-  const size_t b1 = 3 * (size_t)L * o.tiles1 * o.nkb1 * kATile, b2 = 3 * (size_t)L * o.tiles2 * o.nkb2 * kATile;
-  const size_t bs = align256(sizeof(int) * ((size_t)na + m));
-  if (int s = o.buf.ensure(b1 + b2 + bs + sizeof(Norm) * (size_t)nchunk * na)) return s;
+  const CrtPlanes y = planes_of(m, na, L);
+  if (int s = o.buf.ensure(y.total)) return s;
   o.a1 = (int8_t*)o.buf.p;
-  o.a2 = o.a1 + b1;
-  o.s1 = (int*)(o.a2 + b2);
+  o.a2 = o.a1 + y.b1;
+  o.s1 = (int*)(o.a2 + y.b2);
   o.s2 = o.s1 + na;
-  Norm* part = (Norm*)(o.a2 + b2 + bs);
+  Norm* part = (Norm*)(o.a2 + y.b2 + y.bs);
   k_crt_norm_cols<<<dim3(na, nchunk), 256, 0, st>>>(m, na, (const double2*)anl, m, part);
   k_crt_norm_rows<<<(m + 127) / 128, 128, 0, st>>>(m, na, (const double2*)anld, m, pl.beta_a, o.s2);
   with_moduli(L, [&](auto lc) {

@@ -238,10 +238,12 @@ int cpw_b200_hk_psi_spin_device(cpw_b200_ctx* ctx, int neig, const void* psi_sp,
 /* hpsi = H psi for neig device-resident complex128 columns (ld >= mtxd), on
  * `stream` (cudaStream_t; NULL = the context stream). Asynchronous.
  * Same operator as hk_psi_c16.f90:176-231.
- * A call may be captured into a graph after an eager call of the same neig has
- * sized the context's buffers. A replay uses the context's projectors of that
- * moment when they have the captured call's shape; the buffers' addresses are in
- * the graph, so a later call that needs larger ones ends its use. */
+ * Calls of one context share its buffers: the caller orders those of different
+ * streams. A call may be captured into a graph after an eager call of the same
+ * neig, on projectors of the same shape, has sized the buffers. A replay uses the
+ * context's projectors of that moment when they have the captured call's shape;
+ * the buffers' addresses are in the graph, so a later call that needs larger ones
+ * ends its use. */
 int cpw_b200_hk_psi_device(cpw_b200_ctx* ctx, int neig, const void* psi, long long ldpsi, void* hpsi,
                            long long ldhpsi, void* stream);
 /* Local part only, hpsi = V_loc psi (Src/omp/hk_psi_loc_c16.f90 with ladd = .false., nsp = 1). */

@@ -52,3 +52,42 @@ def test_replay_follows_the_projectors(cuda, prec, crt, monkeypatch):
     assert torch.equal(out, eager)
     graph.reset()
     ctx.close()
+
+
+@pytest.mark.parametrize("prec,crt", [(H.FP64, "0"), (H.FP64, "1"), (H.MIXED_TC, "0"), (H.MIXED_TC, "1")])
+def test_capture_before_any_eager_call_with_the_projectors(cuda, prec, crt, monkeypatch):
+    """Buffers sized by other projectors of the shape; the first call with the present ones is the captured one. Eager
+    calls between the capture and the replay see them too."""
+    import torch
+    monkeypatch.setenv("CPW_B200_NL_CRT", crt)
+    d = configs.kpoint_inputs(configs.si2_fcc(), 1)
+    m, na, nb = d["mtxd"], 150, 20
+    rng = np.random.default_rng(8)
+    sets = []
+    for _ in range(3):
+        x = np.asfortranarray(rng.standard_normal((m, na)) + 1j * rng.standard_normal((m, na)))
+        sets.append((x, rng.choice((-1.0, 1.0), na)))
+    ctx = H.Context(0, precision=prec)
+    ctx.set_kpoint(m, d["isort"], d["kgv"], d["ekpg"], d["kmscr"])
+    ctx.set_potential(d["vscr"])
+    psi = torch.randn((nb, m), dtype=torch.complex128, device=cuda).t()
+    out, eager = torch.zeros_like(psi), torch.zeros_like(psi)
+    ctx.set_projectors(*sets[0])
+    ctx.hk_psi(psi, out)
+    ctx.set_projectors(*sets[1])
+    torch.cuda.synchronize()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        ctx.hk_psi(psi, out)
+    ctx.hk_psi(psi, eager)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(out, eager)
+    ctx.set_projectors(*sets[2])
+    graph.replay()
+    torch.cuda.synchronize()
+    ctx.hk_psi(psi, eager)
+    torch.cuda.synchronize()
+    assert torch.equal(out, eager)
+    graph.reset()
+    ctx.close()
