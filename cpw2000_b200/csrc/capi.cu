@@ -201,7 +201,7 @@ int dropin_compute_out(cpw_b200_ctx* c, const DropinPipe& p, double* hpsi, bool 
   // local kernels would be ZGEMMs: 480 bands of Si216 35.1 -> 28.6 ms per call. (Chunks of Si64 with 160 bands do not.)
   int most = 0;
   for (int k = 0; k < p.nchunk; ++k) most = std::max(most, p.start[k + 1] - p.start[k]);
-  const bool split_nl = p.nchunk > 1 && c->nanl > 0 && !(c->precision == 2 && c->tc_ready) &&
+  const bool split_nl = p.nchunk > 1 && c->nanl > 0 && !(c->precision == 2 && (c->tc_ready || c->tc_pending)) &&
                         !ctx_residues(c, most, c->stream);
   if (split_nl) {
     if (int s = dropin_nl_setup(c, p)) return s;

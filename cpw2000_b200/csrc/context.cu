@@ -303,8 +303,7 @@ int ctx_set_projectors(cpw_b200_ctx* c, int nanl, const double* anlga, int ld, c
   e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return cuda_fail(e, "set_projectors");
   if ((s = residues_follow(c))) return s;
-  if (c->precision == 2) return tc_prepare_projectors(c);
-  return kOk;
+  return tc_follow(c);
 }
 
 static int blas_fail(cublasStatus_t st, const char* what) {
@@ -362,12 +361,16 @@ int residues_follow(cpw_b200_ctx* c) {
   return e == cudaSuccess ? kOk : cuda_fail(e, "projector residues");
 }
 
+static bool capturing(cudaStream_t st) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
+  return cap != cudaStreamCaptureStatusNone;
+}
+
 // The residue GEMMs ready for nb bands: X converted, buffers allocated. Where memory does not suffice, or
 // a stream capture forbids the preparation, the products stay on the other path.
 static bool crt_ready(cpw_b200_ctx* c, int nb, cudaStream_t st) {
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(st, &cap) != cudaSuccess) cudaGetLastError();
-  const bool free_run = cap == cudaStreamCaptureStatusNone;
+  const bool free_run = !capturing(st);
   const int L = residue_moduli(c);
   const bool have = c->crt.L == L && c->crt.m == c->mtxd && c->crt.na == c->nanl;
   // projectors that no eager call has converted: the conversion becomes part of the graph
@@ -422,7 +425,10 @@ int ctx_hkpsi_device(cpw_b200_ctx* c, int nb, const void* psi, long long ldpsi, 
   // CPW_B200_NL_OVERLAP=1 / 0 forces either way.
   const bool i8_nl = with_nl && c->nanl > 0 && c->nl_slices > 0;
   const bool crt_nl = with_nl && c->nanl > 0 && !i8_nl && crt_pays(c, nb) && crt_ready(c, nb, st);
-  const bool cublas_nl = with_nl && c->nanl > 0 && !i8_nl && !crt_nl && !(c->precision == 2 && c->tc_ready);
+  const bool tc_nl = with_nl && c->nanl > 0 && !i8_nl && !crt_nl && c->precision == 2 &&
+                     (c->tc_ready || (c->tc_pending && !capturing(st)));
+  if (tc_nl && !c->tc_ready && (s = tc_prepare_projectors(c, st))) return s;
+  const bool cublas_nl = with_nl && c->nanl > 0 && !i8_nl && !crt_nl && !tc_nl;
   bool overlap = false;
   cudaEvent_t ov_t0 = nullptr, ov_t1 = nullptr;
   if (cublas_nl) {
@@ -542,7 +548,7 @@ int ctx_hkpsi_device(cpw_b200_ctx* c, int nb, const void* psi, long long ldpsi, 
       c->timer.mark(kStNlExpand, t1, t2);
       return kOk;
     }
-    if (c->precision == 2 && c->tc_ready) {
+    if (tc_nl) {
       // opt-in mixed form: split-TF32 tensor-core products (nl_tc.cu)
       ++c->forms[kFormSplitTf32];
       if ((s = tc_nl_apply(c, nb, psi, ldpsi, hpsi, ldh, st, t0, t1, t2))) return s;

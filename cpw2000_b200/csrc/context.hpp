@@ -142,7 +142,10 @@ int crt_nl_apply(CrtScratch& t, const CrtOperands& o, int nb, const void* psi, l
                  long long ldh, const TcScratch& tcs, cudaStream_t st, cudaEvent_t t0, cudaEvent_t t1, cudaEvent_t t2);
 int tc_error_flag(TcScratch& t);
 int tc_read_error(TcScratch& t);
-int tc_prepare_projectors(cpw_b200_ctx* c);
+int tc_prepare_projectors(cpw_b200_ctx* c, cudaStream_t st);
+// after new projectors: their split-TF32 operands, unless the set takes residues (then the first block of a solve
+// makes them: 3.4 ms and 32 bytes per element of X for the 216-atom cell)
+int tc_follow(cpw_b200_ctx* c);
 int tc_prepare_operands(int m, int na, const void* anl, const void* anld, DevBuf& a1buf, DevBuf& a2buf,
                         long long* nkb1_out, long long* nkb2_out, cudaStream_t st);
 int tc_nl_apply_ops(TcScratch& t, int m, int na, long long nkb1, long long nkb2, const float* a1, const float* a2,
@@ -214,7 +217,7 @@ struct cpw_b200_ctx {
   bool crt_in_graph = false;    // the call being captured converts the projectors itself
   bool solving = false;         // inside ditsp_device
   long long tc_k1p = 0, tc_k2p = 0;     // K blocks (32 reals) of the projection and expansion operands
-  bool tc_ready = false;
+  bool tc_ready = false, tc_pending = false;      // pending: set in MIXED_TC, not made yet
 
   // two-component spinors (hk_psi_spin_c16): nsp potential combinations scaled by 1/N
   // ([V] or [V1+V2, V1-V2] or [V1+V2, V1-V2, V3, -V4]), the spinor projectors (2 mtxd rows)
@@ -255,7 +258,7 @@ int ctx_set_potential(cpw_b200_ctx* c, const double* vscr, long long nscr);
 int ctx_set_projectors(cpw_b200_ctx* c, int nanl, const double* anlga, int ld, const double* xnlkb, bool on_device);
 // the projectors on the device have changed: what was derived from them is no longer valid
 inline void projectors_changed(cpw_b200_ctx* c) {
-  c->tc_ready = false;
+  c->tc_ready = c->tc_pending = false;
   c->oz_nl_ready = false;
   c->crt.L = 0;
   c->crt_off = false;

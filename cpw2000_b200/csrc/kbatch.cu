@@ -446,6 +446,8 @@ int cpw_b200_kbatch_set_projectors(cpw_b200_kbatch* b, int ik, int nanl, const v
     if ((s = cpwb::tc_prepare_operands(m, nanl, b->anl[ik].p, b->anld[ik].p, b->tca1[ik], b->tca2[ik], &b->nkb1[ik],
                                        &b->nkb2[ik], b->st)))
       return s;
+    const cudaError_t e = cudaStreamSynchronize(b->st);
+    if (e != cudaSuccess) return cuda_fail(e, "kbatch projectors");
     b->tc_ready[ik] = 1;
   }
   // a captured call refers to the old operands

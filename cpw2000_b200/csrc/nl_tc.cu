@@ -566,6 +566,7 @@ int tc_read_error(TcScratch& t) {
   return fail(kTimeout, "tensor-core GEMM: an mbarrier wait gave up");
 }
 
+// the operands' work is queued on st
 int tc_prepare_operands(int m, int na, const void* anl, const void* anld, DevBuf& a1buf, DevBuf& a2buf,
                         long long* nkb1_out, long long* nkb2_out, cudaStream_t st) {
   if (na == 0 || m == 0) return kOk;
@@ -582,20 +583,29 @@ int tc_prepare_operands(int m, int na, const void* anl, const void* anld, DevBuf
   tc::k_prep_a1<<<grid_for(2LL * na * nkb1 * 16, nsm), 256, 0, st>>>(m, na, nkb1, (const C2<double>*)anl, a1, a1 + fa1);
   tc::k_prep_a2<<<grid_for((long long)m * nkb2 * 16, nsm), 256, 0, st>>>(m, na, nkb2, (const C2<double>*)anld, a2,
                                                                           a2 + fa2);
-  cudaError_t e = cudaStreamSynchronize(st);
+  cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, "tensor-core projector preparation");
   *nkb1_out = nkb1;
   *nkb2_out = nkb2;
   return kOk;
 }
 
-int tc_prepare_projectors(cpw_b200_ctx* c) {
+int tc_prepare_projectors(cpw_b200_ctx* c, cudaStream_t st) {
   if (c->nanl == 0 || c->mtxd == 0) return kOk;
-  int s = tc_prepare_operands(c->mtxd, c->nanl, c->anl.p, c->anld.p, c->tc_a1, c->tc_a2, &c->tc_k1p, &c->tc_k2p,
-                              c->stream);
+  int s = tc_prepare_operands(c->mtxd, c->nanl, c->anl.p, c->anld.p, c->tc_a1, c->tc_a2, &c->tc_k1p, &c->tc_k2p, st);
   if (s) return s;
   c->tc_ready = true;
+  c->tc_pending = false;
   return kOk;
+}
+
+int tc_follow(cpw_b200_ctx* c) {
+  if (c->precision != 2) return kOk;
+  c->tc_pending = true;
+  if (residues_pay(c->precision, c->mtxd, c->nanl, 1)) return kOk;
+  if (int s = tc_prepare_projectors(c, c->stream)) return s;
+  const cudaError_t e = cudaStreamSynchronize(c->stream);
+  return e == cudaSuccess ? kOk : cuda_fail(e, "tensor-core projector preparation");
 }
 
 // hpsi += X D X^H psi in split TF32 on the tensor cores (hpsi already holds the local part);

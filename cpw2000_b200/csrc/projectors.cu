@@ -408,8 +408,7 @@ int ctx_proj_nl_kb(cpw_b200_ctx* c, const double* rkpt, int ntype, const int* na
   e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) return cuda_fail(e, "proj_nl_kb");
   if (int s = residues_follow(c)) return s;
-  if (c->precision == 2) return tc_prepare_projectors(c);
-  return kOk;
+  return tc_follow(c);
 }
 
 int ctx_proj_nl_kb_der(cpw_b200_ctx* c, int nder, const double* rkpt, int ntype, const int* natom, const double* rat,

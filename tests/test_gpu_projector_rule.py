@@ -72,6 +72,33 @@ def _forms(cuda, ctx, m, nbs):
     return out
 
 
+def test_split_tf32_of_a_residue_set(cuda, monkeypatch):
+    """Its operands are made by the first block that takes them, and again after new projectors."""
+    import torch
+    d = configs.kpoint_inputs(configs.si8_cubic_kbatch(nk=1), 0)
+    m, na, nb = d["mtxd"], 3600, 5
+    ctx = _context(dict(d, ekpg=0 * d["ekpg"], vscr=0 * d["vscr"]), H.MIXED_TC, na)
+    psi = torch.randn((nb, m), dtype=torch.complex128, device=cuda).t()
+    out = {}
+    for seed in (1, 2):
+        x, xnl = _projectors(m, na, seed)
+        ctx.set_projectors(x, xnl)
+        for form, force in (("residues", None), ("split_tf32", "0"), ("residues", None)):
+            monkeypatch.delenv("CPW_B200_NL_CRT", raising=False)
+            if force:
+                monkeypatch.setenv("CPW_B200_NL_CRT", force)
+            h, before = torch.zeros_like(psi), ctx.form_counts()
+            ctx.hk_psi(psi, h)
+            ctx.synchronize()
+            assert _taken(before, ctx.form_counts()) == {form}
+            p = psi.cpu().numpy()
+            ref = x @ (xnl[:, None] * (x.conj().T @ p))
+            assert np.abs(h.cpu().numpy() - ref).max() < 2e-5 * np.abs(ref).max()
+            out[seed, form] = h
+        assert not torch.equal(out[seed, "residues"], out[seed, "split_tf32"])
+    ctx.close()
+
+
 def test_mixed_tc_form_follows_the_projector_set(cuda):
     """16 M elements of X: below, split TF32 for any number of bands; above, residues."""
     d = configs.kpoint_inputs(configs.si8_cubic_kbatch(nk=1), 0)
