@@ -120,10 +120,11 @@ int oz_read_error(OzScratch& w);
 constexpr int kCrtMaxProjectors = 65535;      // K' of the expansion fits one int32 accumulation
 struct CrtOperands {
   DevBuf buf;
-  int8_t* a1 = nullptr;     // in buf: planes of X and of X D, scales of their rows
+  int8_t* a1 = nullptr;     // in buf: planes of X (balanced) and of X D, scales of their rows
   int8_t* a2 = nullptr;
   int* s1 = nullptr;
   int* s2 = nullptr;
+  double* w = nullptr;      // weights that balance psi, then those of X
   int m = 0, na = 0, L = 0;
   int nkb1 = 0, nkb2 = 0, tiles1 = 0, tiles2 = 0;
   struct Shape {

@@ -9,10 +9,19 @@
 //   * for each modulus p_l the residues (signed bytes) are multiplied with exact int32 accumulation,
 //     so that  sum a b  is known modulo P = p_1 ... p_L;
 //   * |sum a b| <= 2^(beta_a + beta_b) < P / 4 (Cauchy-Schwarz), so the residues determine it.
-// The only error is the rounding of the operands: ~0.4 2^-beta |a| |b| for a row pair, against
-// ~0.3-0.5 2^-53 |a| |b| for a chain of FP64 fused multiply-adds. L = 15 (beta 58) therefore replaces
-// the FP64 ZGEMMs and L = 9 (beta 35) the split-TF32 ones, each with a smaller error than the
-// product it replaces. Results do not depend on the tiling, the K splits or the other bands.
+// The only error is the rounding of the operands, ~0.4 2^-beta |a| |b| for a row pair: it follows the rows'
+// norms, where a ZGEMM's follows sum |a_k b_k|. Projectors fall off with the plane wave's energy by orders of
+// magnitude, so the projection is balanced first: plane wave k of X is divided and that of psi multiplied by the
+// power of two at the norm of X's row k. Then |a| |b| is near sum |a_k b_k| whatever psi weighs, and X is
+// held to 57 (L = 9: 34) bits of numbers of like size. Results do not depend on the tiling, the K splits or the
+// other bands. L = 15 (beta 57 for X and X D, 58 for psi and P) takes the place of the FP64 ZGEMMs, L = 9 (beta 34
+// and 35) that of split TF32. X D X^H psi, 2-norm of the error over that of the result, 26,398 plane waves and 256
+// projectors (ZGEMM, L = 15, split TF32, L = 9):
+//   psi                                  norm-wise                        median over the elements
+//   1 / (1 + ekpg)^2                     1.4e-15 8.2e-16 2.1e-7 6.7e-9    1.3e-15 1.2e-15 2.1e-7 9.5e-9
+//   one plane wave, 1e-6 of the others   1.4e-15 4.6e-16 2.1e-7 2.1e-9    2.0e-15 1.7e-15 2.5e-7 8.2e-9
+//   the highest 30 % of energies alone   1.1e-15 9.4e-16 2.1e-7 7.7e-9    1.1e-15 9.4e-16 2.1e-7 7.7e-9
+// (without the balance 4.4e-12 and 3.8e-5 in the last row, 1.8e-16 and 1.4e-9 in the first).
 //
 // Complex products take three real ones per modulus (exact in residues, where the sums below cannot
 // cancel digits away):
@@ -26,7 +35,7 @@
 // What bounds it: kind::i8 products run at 4,096 multiply-adds per clock and SM here (counted by the
 // tensor pipe's active cycles), so 2.3 P/s over the GPU. 480 bands of a 216-atom cell (88,951 plane
 // waves, 864 projectors): FP64 ZGEMMs 17.0 ms; this form 4.6 ms, of which the two residue GEMMs take
-// 2.9 ms (2.4 P/s: the tensor pipe's rate), the conversion of psi 0.8 + 0.1 ms and the reconstruction
+// 2.9 ms (2.4 P/s: the tensor pipe's rate), the conversion of psi 0.86 + 0.1 ms and the reconstruction
 // 0.75 ms (15 moduli; with 9 in place of split TF32: 5.9 -> 3.1 ms). Four real products per modulus
 // (two rows per complex one) take 3.8 ms in the GEMMs.
 //
@@ -421,9 +430,43 @@ __device__ __forceinline__ int swz8(int r, int c) { return r * KB + (((c >> 1) ^
 
 constexpr int kNormChunk = 4096;       // complex numbers per block of the column norms
 
-// partial norms of the columns of a complex block: part[chunk][ncol]
+// Norms of 32 rows of a complex block (m rows, K columns): a warp takes every kRowThreads / 32-th column of them, warp
+// 0 returns the sum
+constexpr int kRowThreads = 256;
+__device__ __forceinline__ Norm row_norm(int m, int K, const double2* __restrict__ x, long long ldx) {
+  __shared__ Norm sh[kRowThreads];
+  const int lane = threadIdx.x & 31, i = blockIdx.x * 32 + lane;
+  Norm n{0.0, 0.0, 0.0, 0.0};
+  if (i < m) {
+#pragma unroll 8
+    for (int k = threadIdx.x >> 5; k < K; k += kRowThreads / 32) {
+      const double2 v = x[(size_t)k * ldx + i];
+      norm_add(n, v.x);
+      norm_add(n, v.y);
+    }
+  }
+  sh[threadIdx.x] = n;
+  __syncthreads();
+  if (threadIdx.x < 32)
+    for (int t = 1; t < kRowThreads / 32; ++t) n = norm_join(n, sh[32 * t + lane]);
+  return n;
+}
+
+// Weights of the plane waves: w = the power of two above the norm of X's row, and its inverse. Zero where the row is
+// zero (a NaN or an infinity of psi stays one there, as in the product with the zeros).
+__global__ void __launch_bounds__(kRowThreads) k_crt_weights(int m, int K, const double2* __restrict__ x, long long ldx,
+                                                             double* __restrict__ w, double* __restrict__ winv) {
+  const Norm n = row_norm(m, K, x, ldx);
+  const int i = blockIdx.x * 32 + threadIdx.x;
+  if (threadIdx.x >= 32 || i >= m) return;
+  const int s = norm_scale(n, 0), e = s == kNanScale ? 0 : max(-900, min(900, -s));
+  w[i] = n.mx == 0.0 ? 0.0 : pow2(e);
+  winv[i] = n.mx == 0.0 ? 0.0 : pow2(-e);
+}
+
+// partial norms of the columns of a complex block with weighted rows: part[chunk][ncol]
 __global__ void __launch_bounds__(256) k_crt_norm_cols(int m, int ncol, const double2* __restrict__ x, long long ldx,
-                                                       Norm* __restrict__ part) {
+                                                       const double* __restrict__ w, Norm* __restrict__ part) {
   __shared__ Norm sh[32];
   const int col = blockIdx.x, k0 = blockIdx.y * kNormChunk, k1 = min(m, k0 + kNormChunk);
   const double2* c = x + (size_t)col * ldx;
@@ -431,35 +474,30 @@ __global__ void __launch_bounds__(256) k_crt_norm_cols(int m, int ncol, const do
 #pragma unroll 4
   for (int k = k0 + threadIdx.x; k < k1; k += 256) {
     const double2 v = c[k];
-    norm_add(n, v.x);
-    norm_add(n, v.y);
+    const double f = w[k];
+    norm_add(n, v.x * f);
+    norm_add(n, v.y * f);
   }
   n = block_norm(n, sh);
   if (threadIdx.x == 0) part[(size_t)blockIdx.y * ncol + col] = n;
 }
 
-// norms of the rows of a complex block (m rows, K columns): scale exponents
-__global__ void __launch_bounds__(128) k_crt_norm_rows(int m, int K, const double2* __restrict__ x, long long ldx,
-                                                       int beta, int* __restrict__ s) {
-  const int i = blockIdx.x * 128 + threadIdx.x;
-  if (i >= m) return;
-  Norm n{0.0, 0.0, 0.0, 0.0};
-#pragma unroll 8
-  for (int k = 0; k < K; ++k) {
-    const double2 v = x[(size_t)k * ldx + i];
-    norm_add(n, v.x);
-    norm_add(n, v.y);
-  }
-  s[i] = norm_scale(n, beta);
+// the rows' scale exponents
+__global__ void __launch_bounds__(kRowThreads) k_crt_norm_rows(int m, int K, const double2* __restrict__ x,
+                                                               long long ldx, int beta, int* __restrict__ s) {
+  const Norm n = row_norm(m, K, x, ldx);
+  const int i = blockIdx.x * 32 + threadIdx.x;
+  if (threadIdx.x < 32 && i < m) s[i] = norm_scale(n, beta);
 }
 
 // Columns of a complex block along K' (contiguous): column n becomes row n of the three planes. One
 // block converts 2,048 complex numbers of one column, staged through shared memory so that its loads
-// are coalesced (16-byte loads of 8 consecutive numbers per thread would touch 32 lines each).
+// are coalesced (16-byte loads of 8 consecutive numbers per thread would touch 32 lines each). Rows weighted as
+// in the norms (w null: not).
 constexpr int kConvPer = 256 * 8;
 template <int L, bool DIFF>
 __global__ void __launch_bounds__(256) k_crt_conv_cols(int m, int ncol, const double2* __restrict__ x, long long ldx,
-                                                       const Norm* __restrict__ part, int nchunk, int beta, int rows,
+                                                       const double* __restrict__ w, const Norm* __restrict__ part, int nchunk, int beta, int rows,
                                                        int tiles, int nkb, int8_t* __restrict__ out,
                                                        int* __restrict__ sout) {
   __shared__ double2 buf[256 * 9];
@@ -471,7 +509,13 @@ __global__ void __launch_bounds__(256) k_crt_conv_cols(int m, int ncol, const do
 #pragma unroll
   for (int j = 0; j < 8; ++j) {
     const int t = tid + 256 * j, k = k0 + t;
-    buf[(t >> 3) * 9 + (t & 7)] = k < m ? x[(size_t)col * ldx + k] : make_double2(0.0, 0.0);
+    double2 v = k < m ? x[(size_t)col * ldx + k] : make_double2(0.0, 0.0);
+    if (w && k < m) {
+      const double f = w[k];
+      v.x *= f;
+      v.y *= f;
+    }
+    buf[(t >> 3) * 9 + (t & 7)] = v;
   }
   __syncthreads();
   const int ch = (k0 >> 3) + tid, kb = ch >> 4;        // 8-byte piece of the row, its K block
@@ -734,7 +778,7 @@ int num_sms() {
 
 }  // namespace crt
 
-// One buffer: planes of X, planes of X D, row scales of both, partial norms (each cudaMalloc costs a few hundred
+// One buffer: planes of X, planes of X D, row scales of both and weights, partial norms (each cudaMalloc costs a few hundred
 // microseconds). Rows past the last one of a tile stay undefined: what they give is not read.
 struct CrtPlanes {
   size_t b1, b2, bs, total;
@@ -745,7 +789,7 @@ static CrtPlanes planes_of(int m, int na, int L) {
   const size_t row = 3 * (size_t)L * kATile;
   y.b1 = row * ((na + BM - 1) / BM) * ((m + KB - 1) / KB);
   y.b2 = row * ((m + BM - 1) / BM) * ((na + KB - 1) / KB);
-  y.bs = align256(sizeof(int) * ((size_t)na + m));
+  y.bs = align256(sizeof(int) * ((size_t)na + m)) + align256(2 * sizeof(double) * (size_t)m);
   y.total = y.b1 + y.b2 + y.bs + sizeof(Norm) * (size_t)((m + kNormChunk - 1) / kNormChunk) * na;
   return y;
 }
@@ -768,13 +812,15 @@ int crt_prepare(CrtOperands& o, int m, int na, int L, const void* anl, const voi
   o.a2 = o.a1 + y.b1;
   o.s1 = (int*)(o.a2 + y.b2);
   o.s2 = o.s1 + na;
+  o.w = (double*)(o.a2 + y.b2 + align256(sizeof(int) * ((size_t)na + m)));
   Norm* part = (Norm*)(o.a2 + y.b2 + y.bs);
-  k_crt_norm_cols<<<dim3(na, nchunk), 256, 0, st>>>(m, na, (const double2*)anl, m, part);
-  k_crt_norm_rows<<<(m + 127) / 128, 128, 0, st>>>(m, na, (const double2*)anld, m, pl.beta_a, o.s2);
+  k_crt_weights<<<(m + 31) / 32, kRowThreads, 0, st>>>(m, na, (const double2*)anl, m, o.w, o.w + m);
+  k_crt_norm_cols<<<dim3(na, nchunk), 256, 0, st>>>(m, na, (const double2*)anl, m, o.w + m, part);
+  k_crt_norm_rows<<<(m + 31) / 32, kRowThreads, 0, st>>>(m, na, (const double2*)anld, m, pl.beta_a, o.s2);
   with_moduli(L, [&](auto lc) {
     constexpr int LL = decltype(lc)::value;
     k_crt_conv_cols<LL, true><<<dim3((o.nkb1 * KB + kConvPer - 1) / kConvPer, na), 256, 0, st>>>(
-        m, na, (const double2*)anl, m, part, nchunk, pl.beta_a, BM, o.tiles1, o.nkb1, o.a1, o.s1);
+        m, na, (const double2*)anl, m, o.w + m, part, nchunk, pl.beta_a, BM, o.tiles1, o.nkb1, o.a1, o.s1);
     k_crt_conv_rows<LL><<<dim3((m + 15) / 16, o.nkb2), 256, 0, st>>>(m, na, (const double2*)anld, m, o.s2, o.tiles2,
                                                                      o.nkb2, o.a2);
   });
@@ -895,13 +941,13 @@ int crt_nl_apply(CrtScratch& t, const CrtOperands& o, int nb, const void* psi, l
   if (t0) cudaEventRecord(t0, st);
   with_moduli(L, [&](auto lc) {
     constexpr int LL = decltype(lc)::value;
-    k_crt_norm_cols<<<dim3(nb, nchunk), 256, 0, st>>>(m, nb, (const double2*)psi, ldpsi, part);
+    k_crt_norm_cols<<<dim3(nb, nchunk), 256, 0, st>>>(m, nb, (const double2*)psi, ldpsi, o.w, part);
     k_crt_conv_cols<LL, false><<<dim3((o.nkb1 * KB + kConvPer - 1) / kConvPer, nb), 256, 0, st>>>(
-        m, nb, (const double2*)psi, ldpsi, part, nchunk, pl.beta_b, z.nt, z.tn, o.nkb1, b1, sb1);
+        m, nb, (const double2*)psi, ldpsi, o.w, part, nchunk, pl.beta_b, z.nt, z.tn, o.nkb1, b1, sb1);
     if ((e = launch_gemm(g1, nsm, st)) != cudaSuccess) return;
     k_crt_p<LL><<<dim3(o.tiles1, n4), 128, 0, st>>>(pl.w, na, nb, z.nsplit, g1.r, g1.ldr, o.s1, sb1, P, part);
     k_crt_conv_cols<LL, false><<<dim3((o.nkb2 * KB + kConvPer - 1) / kConvPer, nb), 256, 0, st>>>(
-        na, nb, P, na, part, o.tiles1, pl.beta_b, z.nt, z.tn, o.nkb2, b2, sb2);
+        na, nb, P, na, nullptr, part, o.tiles1, pl.beta_b, z.nt, z.tn, o.nkb2, b2, sb2);
     if (t1) cudaEventRecord(t1, st);
     if ((e = launch_gemm(g2, nsm, st)) != cudaSuccess) return;
     k_crt_out<LL><<<dim3(o.tiles2, n4), 128, 0, st>>>(pl.w, m, nb, g2.r, g2.ldr, o.s2, sb2, (double2*)hpsi, ldh);

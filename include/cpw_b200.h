@@ -97,7 +97,9 @@ int cpw_b200_wait_selftest(cpw_b200_ctx* ctx, long long limit_ns, void* stream);
  * conversion, else cuBLAS FP64 ZGEMMs; MIXED_TC: 9 moduli or split-TF32
  * tensor-core GEMMs). The residues of X and X D take 90 (MIXED_TC 54) bytes per
  * element of X beside its own 32, and a call's scratch; they are given back when
- * another allocation of the context fails. 7 slices give
+ * another allocation of the context fails. Their operands are rounded relative to
+ * the norms of X's balanced columns and of the bands (57 and 58 bits, MIXED_TC 34
+ * and 35), which leaves smaller errors than the products they replace. 7 slices give
  * FP64-level products (~2^-48 of the row maxima); 4 give ~2^-27, without the
  * bias of FP32 accumulation (the integer sums are exact). */
 int cpw_b200_set_projector_slices(cpw_b200_ctx* ctx, int slices);

@@ -71,6 +71,24 @@ def test_matches_extended_precision(cuda, prec, cell, na, nb):
     ctx.close()
 
 
+@pytest.mark.parametrize("prec", [H.FP64, H.MIXED_TC])
+def test_bands_that_avoid_the_large_projector_elements(cuda, prec):
+    """Projectors that fall off by ten orders of magnitude over the plane waves, bands that live on the smallest rows
+    alone: the result is as accurate relative to its own size as for any other band (bounds as above: sums over
+    the 60 rows and 60 rows of X to 57 or 34 bits of like numbers)."""
+    d = _basis("si2")
+    m, na = d["mtxd"], 40
+    x, xnl, psi = _random(m, na, 5, 9)
+    x = np.asfortranarray(x * np.logspace(0, -10, m)[:, None])
+    psi[:-60] = 0.0
+    x[-7] = 0.0                             # a plane wave that no projector sees
+    ctx = _context(d, prec, x, xnl)
+    got, ref = _apply(cuda, ctx, psi), _exact(x, xnl, psi)
+    err = np.abs(got - ref).max(axis=1) / np.abs(ref).max(axis=1).clip(1e-300)      # row by row
+    assert float(err.max()) < TOL[prec]
+    ctx.close()
+
+
 def test_scales_and_non_finite_bands(cuda):
     """A band of tiny or huge numbers keeps its relative accuracy; a NaN or an infinity makes its own band
     NaN and leaves the others as they are, to the bit."""
