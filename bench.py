@@ -562,6 +562,7 @@ def run_ours(args, world, rank, local, dist):
             ctx.hk_psi(psi, hpsi)
         barrier()
         evs = [(torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)) for _ in range(steps)]
+        before = ctx.form_counts()
         ctx.timing_begin()
         for a, b in evs:
             a.record()
@@ -570,7 +571,7 @@ def run_ours(args, world, rank, local, dist):
         barrier()
         stages = ctx.timing_end()
         ms = sum(a.elapsed_time(b) for a, b in evs) / steps
-        return ms, stages
+        return ms, stages, {k: n - before[k] for k, n in ctx.form_counts().items()}
 
     hbm, _, peak_kind = measured_peaks()
     psi = torch.from_numpy(np.ascontiguousarray(psi_h.T)).to(dev).t()
@@ -586,9 +587,9 @@ def run_ours(args, world, rank, local, dist):
         ctx.set_slab_budget(8 << 30)
         if slices:
             ctx.set_projector_slices(slices)
-        ms, stages = timed(ctx, psi, hpsi, args.steps, args.warmup)
+        ms, stages, forms = timed(ctx, psi, hpsi, args.steps, args.warmup)
         ctx.synchronize()
-        results[prec_name] = (max_over_ranks(ms), stages)
+        results[prec_name] = (max_over_ranks(ms), stages, forms)
         if prec_name == "fp64":
             hpsi64 = hpsi.clone()
         elif prec_name == "fp64_i8":
@@ -645,9 +646,9 @@ def run_ours(args, world, rank, local, dist):
     e2e_rel = float((got - ref_dev).abs().max() / ref_dev.abs().max())
     del psi_pin, hpsi_pin, got, ref_dev
 
-    ms64, st64 = results["fp64"]
-    msmx, stmx = results["mixed"]
-    mstc, sttc = results["mixed_tc"]
+    ms64, st64, fm64 = results["fp64"]
+    msmx, stmx, _ = results["mixed"]
+    mstc, sttc, _ = results["mixed_tc"]
     value = world * NB / (ms64 / 1e3)
     n1, n2, n3 = (int(v) for v in d["kmscr"][3:6])
     roof64 = roofline_of(st64, args.steps, NB, d, 16, n1 * n2 * n3 * 8, hbm, peak_kind,
@@ -686,11 +687,11 @@ def run_ours(args, world, rank, local, dist):
             "precision": "FP64 pruned FFT + V_loc, projector products in the FP64-accurate int8 tensor-core "
                          "Ozaki GEMM (7 slices; cpw_b200_set_projector_slices)",
             "stages": {k: v[0] / args.steps for k, v in results["fp64_i8"][1].items() if v[1]}},
-        # the residue form of one call's projector products is seven kernels (csrc/crt.cu)
+        # of the timed FP64 calls: the residue form of a call's projector products is seven kernels (csrc/crt.cu),
+        # the other one two library products
         "gpu_launches": int(sum(v[1] for k, v in st64.items() if k in ("inv_xy", "z_vloc", "fwd_xy"))
-                            + (7 * st64["nl_proj"][1] if os.environ.get("CPW_B200_NL_CRT") != "0" else 0)),
-        "library_launches": {"cublas_zgemm": int(st64["nl_proj"][1] + st64["nl_expand"][1])
-                             if os.environ.get("CPW_B200_NL_CRT") == "0" else 0},
+                            + 7 * fm64["residues"]),
+        "library_launches": {"cublas_zgemm": 2 * fm64["zgemm"]},
         "clocks": clocks,
     }
     line["si64"] = si64_throughput(local, max(3, args.steps // 2), 3)
