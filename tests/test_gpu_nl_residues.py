@@ -182,3 +182,21 @@ def test_first_call_on_new_projectors_does_not_wait(cuda, prec):
     ref = _exact(x, xnl, psi)
     assert float(np.abs(h.cpu().numpy() - ref).max() / np.abs(ref).max()) < TOL[prec]
     ctx.close()
+
+
+@pytest.mark.parametrize("prec", [H.FP64, H.MIXED_TC])
+def test_several_accumulations_along_the_plane_waves(cuda, prec):
+    """70,000 plane waves: more than the 512 K blocks of 128 that one int32 accumulation holds. Sums of 2 x 70,000
+    products of operands held to 2^-57 and 2^-34 of their norms: sqrt(140,000) 2^-56 = 5.2e-15 and 4.4e-8 of a
+    typical element, a few of these for the largest of 5 x 3 and 70,000 x 3."""
+    k = np.arange(-23, 24)
+    g = np.stack([a.ravel() for a in np.meshgrid(k, k, k, indexing="ij")])
+    g = np.asfortranarray(g[:, np.argsort((g * g).sum(0), kind="stable")[:70000]].astype(np.int32))
+    m = 70000
+    d = dict(mtxd=m, isort=np.arange(1, m + 1, dtype=np.int32), kgv=g, ekpg=np.zeros(m), vscr=np.zeros(49 * 48 * 48),
+             kmscr=np.array([23, 23, 23, 48, 48, 48, 49], dtype=np.int32))
+    x, xnl, psi = _random(m, 5, 3, 12)
+    ctx = _context(d, prec, x, xnl)
+    got, ref = _apply(cuda, ctx, psi), _exact(x, xnl, psi)
+    assert float(np.abs(got - ref).max() / np.abs(ref).max()) < {H.FP64: 3e-14, H.MIXED_TC: 3e-7}[prec]
+    ctx.close()
