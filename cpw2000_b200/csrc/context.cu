@@ -325,19 +325,20 @@ static int blas_fail(cublasStatus_t st, const char* what) {
 //   9,898, 700: 64 bands 248 -> 211, 459 (ZGEMMs); 160 564 -> 255, 454; 89,137, 200: 96 bands 925 -> 888, 840 (ZGEMMs)
 //   89,137, 64, 480 bands: 1,511 -> 3,019; 34,809, 100, 300 bands: 674 -> 843 (ZGEMMs)
 //
-// MIXED_TC, where the other form is split TF32 and differs by ~1e-7: by the projector set alone, so that a
-// band's result does not depend on the other bands of its call. Sets of kResidueElements elements of X, where
-// residues are no more than 8 % slower at any number of bands (17.8 M elements: 263 -> 240 at 4 bands, 314 ->
-// 337 at 64, 449 -> 440 at 128, 1,033 -> 770 at 270) and the conversion no more than the split (13.7 M: 240 -> 280
-// at 64 bands; 6.8 M: 126 -> 131 at 4, 211 -> 253 at 128, 311 -> 296 at 160; 77 M: 892 -> 702 at 4, 2,961 -> 1,726
-// at 240, conversion 2,300 against 3,400).
+// MIXED_TC, where the other form is split TF32, whose products are ~1e-7 off where residues are ~1e-8: sets of
+// kResidueElements elements of X take residues for any number of bands, so that a band's result does not depend on
+// the other bands of its call. There they are no more than 8 % slower (17.8 M elements: 263 -> 240 at 4 bands, 314
+// -> 337 at 64, 449 -> 440 at 128, 1,033 -> 770 at 270; 77 M: 892 -> 702 at 4, 2,961 -> 1,726 at 240) and converted no
+// slower than split (77 M: 2,300 against 3,400). Smaller sets take them from 128 bands, a full output tile of split
+// TF32, where they need not cost less (6.8 M elements: 126 -> 131 at 4 bands, 211 -> 253 at 128, 311 -> 296 at 160; 13.7
+// M: 240 -> 280 at 64, 356 -> 372 at 128, 643 -> 534 at 225), for their accuracy.
 constexpr double kResidueCalls = 8, kResidueElements = 1.6e7;
 bool residues_pay(int precision, int m, int nanl, int nb) {
   // int32 sums, a grid dimension, 16-bit sums over the K splits
   if (nanl <= 0 || nanl > kCrtMaxProjectors || nb > 65535 || m > 15000000) return false;
   if (const char* v = getenv("CPW_B200_NL_CRT")) return atoi(v) != 0;
   const double elements = (double)m * nanl, waves = (double)m * nb;
-  if (precision == 2) return elements >= kResidueElements;
+  if (precision == 2) return elements >= kResidueElements || (nb >= 128 && 16.0 * elements * nb >= 1.5e10);
   const double zgemm = 16.0 * elements * nb / 33e6, residues = 75 + 15e-6 * elements + 55e-6 * waves;
   return kResidueCalls * (zgemm - residues) >= 50e-6 * elements;
 }

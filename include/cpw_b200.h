@@ -48,9 +48,10 @@ extern "C" {
 /* ---- precision modes ---- */
 #define CPW_B200_FP64 0  /* plain FP64 everywhere (the drop-in default) */
 #define CPW_B200_MIXED 1 /* FP32 FFT/V_loc, FP64 projector GEMMs, FP64 subspace steps */
-/* MIXED with the projector products as split-TF32 (hi.hi + hi.lo + lo.hi) tcgen05 GEMMs with FP32
- * accumulation in tensor memory: ~1e-6 relative error in the projector term; opt-in, set before the
- * projectors (they are prepared in the split layouts at set_projectors). */
+/* MIXED with the projector products as tcgen05 GEMMs: split TF32 (hi.hi + hi.lo + lo.hi, FP32 accumulation in
+ * tensor memory, ~1e-6 relative error in the projector term) or residues with 9 moduli (~1e-8), these for any
+ * number of bands from 16 million elements of X on, else for large blocks (128 bands). A solve takes split TF32
+ * for all its blocks. Opt-in, set before the projectors (their operands are prepared for it). */
 #define CPW_B200_MIXED_TC 2
 
 typedef struct cpw_b200_ctx cpw_b200_ctx;

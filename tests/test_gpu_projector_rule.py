@@ -100,12 +100,14 @@ def test_split_tf32_of_a_residue_set(cuda, monkeypatch):
 
 
 def test_mixed_tc_form_follows_the_projector_set(cuda):
-    """16 M elements of X: below, split TF32 for any number of bands; above, residues."""
+    """From 16 M elements of X on, residues for any number of bands; below, from 128 bands and 15 GFLOP."""
     d = configs.kpoint_inputs(configs.si8_cubic_kbatch(nk=1), 0)
     m = d["mtxd"]
     na = int(1.6e7 / m) + 1
     assert set(_forms(cuda, _context(d, H.MIXED_TC, na), m, (1, 60, 140)).values()) == {"residues"}
-    assert set(_forms(cuda, _context(d, H.MIXED_TC, na - 1), m, (1, 60, 140)).values()) == {"split_tf32"}
+    assert _forms(cuda, _context(d, H.MIXED_TC, na - 1), m, (1, 127, 128)) == {1: "split_tf32", 127: "split_tf32",
+                                                                             128: "residues"}
+    assert _forms(cuda, _context(d, H.MIXED_TC, 1500), m, (128, 140)) == {128: "split_tf32", 140: "residues"}
 
 
 @pytest.mark.parametrize("na,nb,form", [(700, 60, "zgemm"), (700, 200, "residues"), (32, 400, "zgemm"),
