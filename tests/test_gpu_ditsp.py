@@ -65,7 +65,8 @@ def test_ditsp_fp64_matches_dense_truth_and_oracle(cuda, ik):
 
 @pytest.mark.parametrize("prec", [H.MIXED, H.MIXED_TC])
 def test_ditsp_mixed_within_1e6(cuda, prec):
-    """Mixed form (FP32 local part; MIXED_TC also split-TF32 projector products and Ritz rotations;
+    """Mixed form (FP32 local part; MIXED_TC also split-TF32 projector products, for every block of a solve, and Ritz
+    rotations;
     both with Cholesky QR in-block orthonormalisation) within 1e-6 Ha of dense truth."""
     import torch
     w = configs.si2_fcc()
