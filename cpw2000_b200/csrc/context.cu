@@ -373,6 +373,8 @@ static bool capturing(cudaStream_t st) {
 static bool crt_ready(cpw_b200_ctx* c, int nb, cudaStream_t st) {
   const bool free_run = !capturing(st);
   const int L = residue_moduli(c);
+  if (c->crt_in_graph) c->crt.L = 0;      // planes that only a replay of that graph has
+  c->crt_in_graph = false;
   const bool have = c->crt.L == L && c->crt.m == c->mtxd && c->crt.na == c->nanl;
   // projectors that no eager call has converted: the conversion becomes part of the graph
   if (!have && !free_run && c->crt.buf.bytes < crt_plane_bytes(c->mtxd, c->nanl, L)) return false;
@@ -381,6 +383,7 @@ static bool crt_ready(cpw_b200_ctx* c, int nb, cudaStream_t st) {
     ~Making() { c->crt_making = false; }
   } making{c};
   c->crt_making = true;
+  c->crt_in_graph = !have && !free_run;
   if ((!have && crt_prepare(c->crt, c->mtxd, c->nanl, L, c->anl.p, c->anld.p, st)) ||
       crt_reserve(c->crts, c->crt, nb, free_run) || (free_run ? tc_error_flag(c->tcs) != kOk : !c->tcs.err.p)) {
     if (free_run) {
@@ -395,7 +398,6 @@ static bool crt_ready(cpw_b200_ctx* c, int nb, cudaStream_t st) {
   const CrtOperands::Shape now{c->mtxd, c->nanl, L};
   auto& used = c->crt.captured;
   if (!free_run && std::find(used.begin(), used.end(), now) == used.end()) used.push_back(now);
-  c->crt_in_graph = !have && !free_run;
   return true;
 }
 
@@ -513,9 +515,7 @@ int ctx_hkpsi_device(cpw_b200_ctx* c, int nb, const void* psi, long long ldpsi, 
     cudaEvent_t t0 = c->timer.on ? c->timer.take() : nullptr, t1 = c->timer.on ? c->timer.take() : nullptr;
     cudaEvent_t t2 = c->timer.on ? c->timer.take() : nullptr;
     ++c->forms[kFormResidues];
-    s = crt_nl_apply(c->crts, c->crt, nb, psi, ldpsi, hpsi, ldh, c->tcs, st, t0, t1, t2);
-    if (c->crt_in_graph) c->crt.L = 0;          // only a replay has the planes
-    if (s) return s;
+    if ((s = crt_nl_apply(c->crts, c->crt, nb, psi, ldpsi, hpsi, ldh, c->tcs, st, t0, t1, t2))) return s;
     c->timer.mark(kStNlProj, t0, t1);
     c->timer.mark(kStNlExpand, t1, t2);
     return kOk;

@@ -215,7 +215,7 @@ struct cpw_b200_ctx {
   cpwb::CrtScratch crts;
   bool crt_off = false;
   bool crt_making = false;      // being made: not to be taken back
-  bool crt_in_graph = false;    // the call being captured converts the projectors itself
+  bool crt_in_graph = false;    // the last conversion was captured, not run
   bool solving = false;         // inside ditsp_device
   long long tc_k1p = 0, tc_k2p = 0;     // K blocks (32 reals) of the projection and expansion operands
   bool tc_ready = false, tc_pending = false;      // pending: set in MIXED_TC, not made yet
@@ -262,6 +262,7 @@ inline void projectors_changed(cpw_b200_ctx* c) {
   c->tc_ready = c->tc_pending = false;
   c->oz_nl_ready = false;
   c->crt.L = 0;
+  c->crt_in_graph = false;
   c->crt_off = false;
 }
 void ditsp_release(cpw_b200_ctx* c);

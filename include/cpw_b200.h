@@ -75,9 +75,9 @@ int cpw_b200_set_slab_budget(cpw_b200_ctx* ctx, long long bytes);
 
 /* Bounded device waits (failure detection). Every wait of this library's kernels
  * on another party gives up after a limit, records the failure and lets the
- * kernel return; the host then reports CPW_B200_TIMEOUT (from
- * cpw_b200_synchronize for the tensor-core GEMMs, from the eigensolver call for
- * its cooperative Gram-Schmidt kernel) and the context stays usable.
+ * kernel return; the host then reports CPW_B200_TIMEOUT (for the tensor-core
+ * GEMMs from cpw_b200_synchronize, the drop-ins and the eigensolver, for the
+ * eigensolver's Gram-Schmidt kernels from its call) and the context stays usable.
  * set_wait_limits: the time limit of the tensor-core GEMMs' hand-off mbarrier
  *   waits (default 2 s) and the poll limit of the Gram-Schmidt grid barrier
  *   (default 2^24, ~1 s); a negative value restores the default. The waits for

@@ -8,6 +8,7 @@ import pytest
 
 from cpw2000_b200 import configs
 from cpw2000_b200 import hk_psi as H
+from cpw2000_b200._lib import CpwB200Error
 
 pytestmark = pytest.mark.gpu
 
@@ -90,4 +91,46 @@ def test_capture_before_any_eager_call_with_the_projectors(cuda, prec, crt, monk
     torch.cuda.synchronize()
     assert torch.equal(out, eager)
     graph.reset()
+    ctx.close()
+
+
+@pytest.mark.parametrize("prec", [H.FP64, H.MIXED_TC])
+def test_a_discarded_capture_leaves_no_planes_behind(cuda, prec, monkeypatch):
+    """New projectors, then a captured call that needs more scratch than any eager call has sized, thrown away: what
+    it recorded of the conversion never ran. The next eager call converts for itself."""
+    import ctypes as C
+
+    import torch
+    rt = C.CDLL("libcudart.so.12")
+    monkeypatch.setenv("CPW_B200_NL_CRT", "1")
+    d = configs.kpoint_inputs(configs.si2_fcc(), 1)
+    m, na, nb = d["mtxd"], 150, 300
+    rng = np.random.default_rng(9)
+    x = [np.asfortranarray(rng.standard_normal((m, na)) + 1j * rng.standard_normal((m, na))) for _ in range(2)]
+    xnl = rng.choice((-1.0, 1.0), na)
+    ctx = H.Context(0, precision=prec)
+    ctx.set_kpoint(m, d["isort"], d["kgv"], 0 * d["ekpg"], d["kmscr"])
+    ctx.set_potential(0 * d["vscr"])
+    ctx.set_slab_budget(1)                  # one band at a time: the slab does not grow
+    psi = torch.randn((nb, m), dtype=torch.complex128, device=cuda).t()
+    out = torch.zeros_like(psi)
+    ctx.set_projectors(x[0], xnl)
+    ctx.hk_psi(psi, out, neig=20)
+    ctx.set_projectors(x[1], xnl)
+    torch.cuda.synchronize()
+    st, graph = torch.cuda.Stream(), C.c_void_p()
+    assert rt.cudaStreamBeginCapture(C.c_void_p(st.cuda_stream), 2) == 0        # relaxed: allocations may go on
+    try:
+        ctx.hk_psi(psi, out, stream=st.cuda_stream)
+    except CpwB200Error:
+        pass
+    rt.cudaStreamEndCapture(C.c_void_p(st.cuda_stream), C.byref(graph))
+    if graph:
+        assert rt.cudaGraphDestroy(graph) == 0
+    torch.cuda.synchronize()
+    ctx.hk_psi(psi, out)
+    ctx.synchronize()
+    p = psi.cpu().numpy()
+    ref = x[1] @ (xnl[:, None] * (x[1].conj().T @ p))
+    assert np.abs(out.cpu().numpy() - ref).max() < (1e-12 if prec == H.FP64 else 1e-6) * np.abs(ref).max()
     ctx.close()
