@@ -12,9 +12,6 @@
 #include "../../include/cpw_b200.h"
 #include "context.hpp"
 
-namespace cpwb {
-}
-
 using namespace cpwb;
 using C2d = C2<double>;
 

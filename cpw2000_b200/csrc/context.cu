@@ -330,8 +330,8 @@ static int blas_fail(cublasStatus_t st, const char* what) {
 // the other bands of its call. There they are no more than 8 % slower (17.8 M elements: 263 -> 240 at 4 bands, 314
 // -> 337 at 64, 449 -> 440 at 128, 1,033 -> 770 at 270; 77 M: 892 -> 702 at 4, 2,961 -> 1,726 at 240) and converted no
 // slower than split (77 M: 2,300 against 3,400). Smaller sets take them from 128 bands, a full output tile of split
-// TF32, where they need not cost less (6.8 M elements: 126 -> 131 at 4 bands, 211 -> 253 at 128, 311 -> 296 at 160; 13.7
-// M: 240 -> 280 at 64, 356 -> 372 at 128, 643 -> 534 at 225), for their accuracy.
+// TF32, where they need not cost less (6.8 M elements: 126 -> 131 at 4 bands, 211 -> 253 at 128, 311 -> 296 at 160;
+// 13.7 M: 240 -> 280 at 64, 356 -> 372 at 128, 643 -> 534 at 225), for their accuracy.
 constexpr double kResidueCalls = 8, kResidueElements = 1.6e7;
 bool residues_pay(int precision, int m, int nanl, int nb) {
   // int32 sums, a grid dimension, 16-bit sums over the K splits

@@ -30,7 +30,15 @@ enum Status : int {
 // enabled; read back (with one synchronisation) by timing_end.
 enum Stage : int { kStInvXY = 0, kStZVloc = 1, kStFwdXY = 2, kStNlProj = 3, kStNlExpand = 4, kStEig = 5, kNumStages = 8 };
 // Forms that the host code chooses between by size, counted per call (cpw_b200_form_counts)
-enum Form : int { kFormZgemm = 0, kFormSplitTf32 = 1, kFormResidues = 2, kFormSlices = 3, kFormMgsCluster = 4, kFormMgsGrid = 5, kNumForms = 6 };
+enum Form : int {
+  kFormZgemm = 0,
+  kFormSplitTf32 = 1,
+  kFormResidues = 2,
+  kFormSlices = 3,
+  kFormMgsCluster = 4,
+  kFormMgsGrid = 5,
+  kNumForms = 6
+};
 struct StageTimer {
   bool on = false;
   std::vector<cudaEvent_t> pool;

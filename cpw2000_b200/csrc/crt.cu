@@ -497,9 +497,9 @@ __global__ void __launch_bounds__(kRowThreads) k_crt_norm_rows(int m, int K, con
 constexpr int kConvPer = 256 * 8;
 template <int L, bool DIFF>
 __global__ void __launch_bounds__(256) k_crt_conv_cols(int m, int ncol, const double2* __restrict__ x, long long ldx,
-                                                       const double* __restrict__ w, const Norm* __restrict__ part, int nchunk, int beta, int rows,
-                                                       int tiles, int nkb, int8_t* __restrict__ out,
-                                                       int* __restrict__ sout) {
+                                                       const double* __restrict__ w, const Norm* __restrict__ part,
+                                                       int nchunk, int beta, int rows, int tiles, int nkb,
+                                                       int8_t* __restrict__ out, int* __restrict__ sout) {
   __shared__ double2 buf[256 * 9];
   const int col = blockIdx.y, k0 = blockIdx.x * kConvPer, tid = threadIdx.x;
   Norm n{0.0, 0.0, 0.0, 0.0};
@@ -778,8 +778,8 @@ int num_sms() {
 
 }  // namespace crt
 
-// One buffer: planes of X, planes of X D, row scales of both and weights, partial norms (each cudaMalloc costs a few hundred
-// microseconds). Rows past the last one of a tile stay undefined: what they give is not read.
+// One buffer: planes of X, planes of X D, row scales of both and weights, partial norms (each cudaMalloc costs a
+// few hundred microseconds). Rows past the last one of a tile stay undefined: what they give is not read.
 struct CrtPlanes {
   size_t b1, b2, bs, total;
 };
